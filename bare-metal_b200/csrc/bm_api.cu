@@ -6,6 +6,7 @@
 #include "host_common.cuh"
 #include "igemm_dense.cuh"
 #include "igemm_dense_pair.cuh"
+#include "igemm_dense_decode.cuh"
 #include "igemm_sparse.cuh"
 #include "igemm_sparse_pair.cuh"
 #include "pack_kernels.cuh"
@@ -72,6 +73,83 @@ static int launch_dense_bn(int bn, const CUtensorMap& ma, const CUtensorMap& mb,
     }
 }
 
+// Few tokens, weights [N x K]: geometry of the channels-on-lanes kernel and what it should cost.
+struct DenseDecodePlan {
+    int tile_rows, fold;
+    float us;
+};
+// The fewest tiles per SM that fit, and the fold that needs the least tensor time.  `us` is a fit to W8A8 fp16-output
+// runs with 1 to 256 tokens over weights from 512 x 4096 to 28672 x 8192 (within ~20 %): launch, ramp and drain 3.6 us; the
+// weights at 5.9 TB/s or the MMAs (57 clocks each at least, half a clock per column from 114 columns up); on top the
+// activations, which every tile reads again out of L2, at 80 KB/us and SM, and the drain of the tokens.
+static DenseDecodePlan plan_dense_decode(int M, int N, int K, int sms) {
+    const int bn = (M + 15) / 16 * 16, k_chunks = ceil_div(K, kBK);
+    const int groups = ceil_div(N, 8);                                           // channels in groups of 8
+    const int waves = ceil_div(groups, kBM / 8 * sms);
+    const int rows = ceil_div(groups, waves * sms) * 8;
+    DenseDecodePlan plan{rows, 1, 0.f};
+    float mma = 0.f;
+    for (int fold = 1; fold <= 8; fold *= 2) {
+        if (fold > 1 && (rows * fold > kBM || bn * fold > 256 || rows * fold * bn > kDdPartInts || fold > k_chunks)) break;
+        const float us = static_cast<float>(waves) * ceil_div(k_chunks, fold) * 4.f *
+                         (bn * fold < 114 ? 57.f : bn * fold / 2.f) / 1.8e3f;
+        if (fold == 1 || us < mma) { mma = us; plan.fold = fold; }
+    }
+    const float hbm = static_cast<float>(N) * K / 5.9e6f;
+    plan.us = 3.6f + (hbm > mma ? hbm : mma) + (M > 16 ? static_cast<float>(waves) * bn * K / 80e3f + 0.02f * M : 0.f);
+    return plan;
+}
+
+template <int EPI>
+static int launch_dense_decode(const CUtensorMap& w3, const CUtensorMap& w2, const CUtensorMap& x3, const CUtensorMap& x2,
+                               const DenseDecodeParams& p, int grid, cudaStream_t stream) {
+    auto kern = igemm_dense_decode_kernel<EPI>;
+    static ConfiguredFlags flags;
+    if (int rc = ensure_smem_limit(flags, kern, kDdSmemBytes)) return rc;
+    BM_CUDA_TRY(launch_pdl(kern, dim3(grid), dim3(kDdThreads), kDdSmemBytes, stream, 1, w3, w2, x3, x2, p));
+    return BM_OK;
+}
+
+static int dense_decode(int epi, const int8_t* X, const int8_t* W, const EpilogueParams& ep, int M, int N, int K,
+                        const DenseDecodePlan& plan, DeviceState* dev, cudaStream_t stream) {
+    DenseDecodeParams p{};
+    p.epi = ep;
+    p.tile_rows = plan.tile_rows;
+    p.tiles = ceil_div(N, plan.tile_rows);
+    p.tokens_padded = (M + 15) / 16 * 16;
+    p.fold = plan.fold;
+    p.acc_stride = (p.tokens_padded * p.fold + 31) / 32 * 32;
+    p.tmem_cols = 64;
+    while (p.tmem_cols < 2 * p.acc_stride) p.tmem_cols *= 2;
+    const int k_chunks = ceil_div(K, kBK), group_bytes = (p.tile_rows + p.tokens_padded) * kBK * p.fold;
+    p.full_chunks = K / kBK;
+    p.whole_chunks = K % kBK == 0;
+    int per_stage = ceil_div(16 * 1024, group_bytes);            // stages of at least 16 KiB
+    if (per_stage > ceil_div(k_chunks, p.fold)) per_stage = ceil_div(k_chunks, p.fold);
+    p.chunks = per_stage * p.fold;
+    p.stages = kDdRingBytes / (per_stage * group_bytes);
+    if (p.stages > kDdMaxStages) p.stages = kDdMaxStages;
+    p.k_stages = ceil_div(k_chunks, p.chunks);
+    p.status = dev->status;
+    CUtensorMap w2, x2, w3, x3;
+    if (int rc = make_tensor_map_u8(&w2, W, K, N, K, kBK, p.tile_rows, true)) return rc;
+    if (int rc = make_tensor_map_u8(&x2, X, K, M, K, kBK, p.tokens_padded, true)) return rc;
+    w3 = w2;
+    x3 = x2;
+    if (p.whole_chunks || p.full_chunks >= p.chunks) {            // else every stage takes the 2-D maps
+        if (int rc = make_tensor_map_kblocks(&w3, W, p.full_chunks, N, K, p.tile_rows, p.chunks)) return rc;
+        if (int rc = make_tensor_map_kblocks(&x3, X, p.full_chunks, M, K, p.tokens_padded, p.chunks)) return rc;
+    }
+    const int grid = p.tiles < dev->sm_count ? p.tiles : dev->sm_count;
+    switch (epi) {
+        case EPI_I32: return launch_dense_decode<EPI_I32>(w3, w2, x3, x2, p, grid, stream);
+        case EPI_F32_TENSOR: return launch_dense_decode<EPI_F32_TENSOR>(w3, w2, x3, x2, p, grid, stream);
+        case EPI_F32_CHANNEL: return launch_dense_decode<EPI_F32_CHANNEL>(w3, w2, x3, x2, p, grid, stream);
+        case EPI_F16_ROWCOL: return launch_dense_decode<EPI_F16_ROWCOL>(w3, w2, x3, x2, p, grid, stream);
+    }
+    return fail_msg(BM_ERR_LAYOUT, "unknown epilogue");
+}
+
 static int dense_gemm(int epi, const int8_t* A, const int8_t* B, void* C, int M, int N, int K, long long ldc,
                       int b_layout, float tensor_scale, const float* row_scale, const float* col_scale,
                       const int* col_zero, void* stream_v, void* const* peers = nullptr, int n_peers = 0,
@@ -89,8 +167,20 @@ static int dense_gemm(int epi, const int8_t* A, const int8_t* B, void* C, int M,
     if (int rc = current_device_state(&dev)) return rc;
 
     const bool b_mn = (b_layout == BM_B_KN);
+    DenseParams p{};
+    p.epi.out = C;
+    p.epi.ld = ldc;
+    p.epi.rows = M;
+    p.epi.cols = N;
+    p.epi.tensor_scale = tensor_scale;
+    p.epi.row_scale = row_scale;
+    p.epi.col_scale = col_scale;
+    p.epi.col_zero = col_zero;
+    p.epi.vec_ok = aligned16(C) && (static_cast<size_t>(ldc) * out_elem_size(epi)) % 16 == 0;
     const int tiles_m = ceil_div(M, kBM);
     int bn = forced_bn();
+    const bool bn_forced = bn != 0;
+    float tile_us = 0.f;                                 // what the model expects of the chosen tiles
     bool pair_ok = pair_enabled() && dev->sm_count >= 2;
     if (bn == 0) {
         // Tile choice by a wave count model: cost = start-up + waves x (time of one tile per 4096 of K).
@@ -108,9 +198,24 @@ static int dense_gemm(int epi, const int8_t* A, const int8_t* B, void* C, int M,
             const long long tiles = static_cast<long long>(ceil_div(M, c.pair ? 256 : kBM)) * ceil_div(N, c.bn);
             const long long slots = c.pair ? dev->sm_count / 2 : dev->sm_count;
             const float cost = c.start_us + static_cast<float>((tiles + slots - 1) / slots) * c.wave_us;
-            if (bn == 0 || cost < best) { best = cost; bn = c.bn; best_pair = c.pair; }
+            if (bn == 0 || cost < best) {
+                best = cost; bn = c.bn; best_pair = c.pair;
+                tile_us = c.start_us + (cost - c.start_us) * (K / 4096.f);
+            }
         }
         pair_ok = best_pair;
+    }
+    // Few tokens on weights [N x K]: channels on the lanes.  Up to 16 tokens always (the wide tiles spend 11 to 36 us
+    // on zero-filled token rows: 4096 x 4096, 16 tokens 14.4 -> 7.0 us; 12288 x 4096 20.3 -> 12.6; 22016 x 4096
+    // 32.0 -> 22.2; 4096 x 11008 25.0 -> 12.1), above that where the model sees it ahead (4096 x 11008, 32 tokens 25.1 -> 12.3
+    // and 96 tokens 25.4 -> 20.7; but 12288 x 4096, 64 tokens 13.3 against 14.9, and 1024 x 1024 4.3 against 5.5).  The wide
+    // tiles cannot beat the weights' own streaming time either: 22016 x 4096, 32 tokens 21.4 us for 1 wave of 12.3.
+    if (!b_mn && n_peers == 0 && M <= kDdMaxTokens && epi != EPI_F32_ROWCOL && opt(OPT_DENSE_DECODE) != 0) {
+        const DenseDecodePlan plan = plan_dense_decode(M, N, K, dev->sm_count);
+        const float stream_us = 2.6f + 1.15f * N * K / 5.9e6f;
+        const float wide_us = tile_us > stream_us ? tile_us : stream_us;
+        if (opt(OPT_DENSE_DECODE) == 1 || (!bn_forced && (M <= 16 || plan.us < wide_us)))
+            return dense_decode(epi, A, B, p.epi, M, N, K, plan, dev, static_cast<cudaStream_t>(stream_v));
     }
     if (b_mn && bn < 128) bn = 128;
     if (n_peers > 0 && bn < 128) bn = 128;          // the gather rides on the TMA-store epilogue (tiles >= 128 wide)
@@ -125,16 +230,6 @@ static int dense_gemm(int epi, const int8_t* A, const int8_t* B, void* C, int M,
         if (int rc = make_tensor_map_u8(&map_b, B, K, N, K, kBK, use_pair ? kPairHalfN : bn, true)) return rc;
     }
 
-    DenseParams p{};
-    p.epi.out = C;
-    p.epi.ld = ldc;
-    p.epi.rows = M;
-    p.epi.cols = N;
-    p.epi.tensor_scale = tensor_scale;
-    p.epi.row_scale = row_scale;
-    p.epi.col_scale = col_scale;
-    p.epi.col_zero = col_zero;
-    p.epi.vec_ok = aligned16(C) && (static_cast<size_t>(ldc) * out_elem_size(epi)) % 16 == 0;
     OutMaps map_out{};
     p.n_out = 1;
     if (n_peers > 0) {

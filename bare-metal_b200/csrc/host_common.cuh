@@ -52,6 +52,7 @@ enum : int {
     OPT_TAIL_NARROW,         // 0 switches the half-height tiles of a partly filled last wave off
     OPT_PDL,                 // 0 launches without programmatic stream serialization
     OPT_GATHER_GBS,          // fused all-gather: GB/s of peer stores a GPU may send (0 = unpaced)
+    OPT_DENSE_DECODE,        // few tokens: -1 automatic, 0 never, 1 always the channels-on-lanes kernel (where it applies)
     OPT_DECODE_TILE_ROWS,    // row-balanced decode tiles: rows per ring stage (0 automatic; 32 / 64 / 128 pins it)
     OPT_COUNT
 };
@@ -63,7 +64,7 @@ inline const OptionSpec* option_specs() {
         {"tma_store", "BM_TMA_STORE", 1},         {"dense_group_m", "BM_DENSE_GROUP_M", -1},
         {"sparse_col_first", "BM_SPARSE_COL_FIRST", -1}, {"tail_narrow", "BM_TAIL_NARROW", 1},
         {"pdl", "BM_PDL", 1},                     {"gather_gbs", "BM_GATHER_GBS", 680},
-        {"decode_tile_rows", "BM_DECODE_TILE_ROWS", 0},
+        {"dense_decode", "BM_DENSE_DECODE", -1},  {"decode_tile_rows", "BM_DECODE_TILE_ROWS", 0},
     };
     return specs;
 }
@@ -211,7 +212,7 @@ inline MapCache& map_cache() {
 }
 
 // Encodes (or fetches) a tiled map of rank 2 or 3.  dims / box are innermost first; `pitch` is the byte
-// stride of dimension 1 for rank 2, of dimension 2 for rank 3 (dimension 1 of a rank-3 map is 128 bytes).
+// stride of dimension 1; dimension 2 of a rank-3 map steps by 128 bytes (K blocks of a row-major operand).
 inline int cached_tensor_map(CUtensorMap* map, const void* base, int rank, CUtensorMapDataType type, int elem_size,
                              const uint64_t (&dims)[3], uint64_t pitch, const uint32_t (&box)[3], bool swizzle128,
                              bool l2_promote) {
@@ -231,8 +232,7 @@ inline int cached_tensor_map(CUtensorMap* map, const void* base, int rank, CUten
         }
     }
     cuuint64_t gdims[3] = {dims[0], dims[1], dims[2]};
-    cuuint64_t strides[2] = {pitch, 0};
-    if (rank == 3) { strides[0] = 128; strides[1] = pitch; }
+    cuuint64_t strides[2] = {pitch, 128};
     cuuint32_t gbox[3] = {box[0], box[1], box[2]};
     cuuint32_t elem_strides[3] = {1, 1, 1};
     CUresult r = fn(map, type, static_cast<cuuint32_t>(rank), const_cast<void*>(base), gdims, strides, gbox, elem_strides,
@@ -257,6 +257,15 @@ inline int make_tensor_map_u8(CUtensorMap* map, const void* base, uint64_t cols,
     const uint64_t dims[3] = {cols, rows, 1};
     const uint32_t box[3] = {box_cols, box_rows, 1};
     return cached_tensor_map(map, base, 2, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, dims, pitch, box, swizzle128, true);
+}
+
+// K-major byte matrix [rows x K] seen as [k_blocks][rows][128 bytes]: one box holds `box_blocks` K blocks of box_rows
+// rows, each block in the layout a 128 x box_rows box of make_tensor_map_u8 leaves.  Whole K blocks only.
+inline int make_tensor_map_kblocks(CUtensorMap* map, const void* base, uint64_t k_blocks, uint64_t rows, uint64_t pitch,
+                                   uint32_t box_rows, uint32_t box_blocks) {
+    const uint64_t dims[3] = {128, rows, k_blocks};
+    const uint32_t box[3] = {128, box_rows, box_blocks};
+    return cached_tensor_map(map, base, 3, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, dims, pitch, box, true, true);
 }
 
 // Output matrix [rows x cols] of 2- or 4-byte elements for TMA stores: box = 128 bytes x 32 rows,

@@ -253,6 +253,8 @@ int bm_last_device_status(int *code);
  * 0 = choose), "dense_pair", "sparse_pair" (0 = single-CTA kernels only), "row_balanced"
  * (0 = whole 128-row tiles on the decode shapes), "tma_store" (0 = direct-store epilogue),
  * "dense_group_m", "sparse_col_first" (-1 automatic), "tail_narrow", "pdl", "gather_gbs",
+ * "dense_decode" (dense weights [N x K], at most 256 tokens: -1 choose, 0 never / 1 always the kernel with
+ * channels on the lanes),
  * "decode_tile_rows" (row-balanced decode tiles on packed weights: 0 = choose the ring-stage height
  * from the rows a CTA is dealt, 32 / 64 / 128 pins it).
  * Each starts from the environment variable BM_<NAME> read once at first use, else its default;
