@@ -391,7 +391,7 @@ static int launch_sparse_pair(const CUtensorMap& mw, const CUtensorMap& me, cons
     return BM_OK;                                   // (no output tensor map in this orientation: mw fills the slot)
 }
 
-// the reference orientation (sparse operand on the left, B[K x C]) on CTA pairs: 256 rows x 224 columns
+// the reference orientation (sparse operand on the left, B[K x C]) on CTA pairs: 256 rows x 256 columns
 template <int EPI, bool F16>
 static int launch_sparse_pair_left(const CUtensorMap& mw, const CUtensorMap& me, const CUtensorMap& mx,
                                    const CUtensorMap& mo, const SparseParams& p, int pairs, cudaStream_t stream) {
@@ -445,15 +445,18 @@ static int sparse_pair_left(int epi, bool f16, const void* S_comp, const uint8_t
     return fail_msg(BM_ERR_LAYOUT, "unsupported epilogue for the sparse pair kernel");
 }
 
-// When the reference orientation runs on CTA pairs.  Measured against the lone-CTA kernel with 128-column
-// tiles: int8 is no faster on pairs (4096^3: 67.6 vs 58.4 us; 8192^3: 395 vs 371 us), so pairs are used
-// for int8 only when the tile width is forced to 224; fp16 gains 6-18 % once there are two waves of pair tiles
-// (4096^3: 90.7 vs 96.4 us; 8192 x 8192 x 4096: 315 vs 370 us).
-static bool sparse_pair_left_wanted(int R, int Cn, const DeviceState* dev, int forced, bool f16) {
+// When the reference orientation runs on CTA pairs (256 x 256 tiles) instead of lone CTAs (128 x 128): by waves.  One wave of
+// pair tiles takes about 1.4 lone ones (per 4096 of K: int8 11.1 against 7.9 us, fp16 16.8 against 12.4), so
+// pairs win wherever they need fewer than 5/7 of the waves.  Lone CTAs -> pairs: 2048 x 2048 x 2048 (2 waves against 1) int8
+// 14.9 -> 12.0 us, fp16 18.2 -> 12.2; 2048 x 4096 x 4096 (4, 2) 35.7 -> 26.1, 53.7 -> 37.6; 8192^3 (28, 14) 441 -> 313,
+// 890 -> 602; but 1024 x 2048 x 4096 (1, 1) 13.7 -> 14.5, 16.4 -> 16.8.  Tile width 224 forces pairs.
+static bool sparse_pair_left_wanted(int R, int Cn, const DeviceState* dev, int forced) {
     if (forced == 224) return dev->sm_count >= 2;
-    if (forced != 0 || dev->sm_count < 2 || !f16) return false;
-    if (opt(OPT_SPARSE_PAIR) == 0) return false;
-    return static_cast<long long>(ceil_div(R, 256)) * ceil_div(Cn, SpPairCfg<true>::BN) >= dev->sm_count;
+    if (forced != 0 || dev->sm_count < 2 || opt(OPT_SPARSE_PAIR) == 0) return false;
+    auto waves = [&](int rows, int cols, int slots) {
+        return (static_cast<long long>(ceil_div(R, rows)) * ceil_div(Cn, cols) + slots - 1) / slots;
+    };
+    return 7 * waves(256, SpPairCfg<true>::BN, dev->sm_count / 2) < 5 * waves(128, 128, dev->sm_count);
 }
 
 // option "sparse_pair" = 0 keeps large sparse-weight problems on the single-CTA kernel (testing hook)
@@ -520,7 +523,7 @@ static int sparse_gemm(int mode, int epi, const int8_t* S_comp, const uint8_t* m
         return fail_msg(BM_ERR_LAYOUT, "unsupported epilogue for the sparse pair kernel");
     }
     if (bn == 240) bn = 0;
-    if (mode == 0 && dense_mn && !packed && sparse_pair_left_wanted(R, Cn, dev, bn, false))
+    if (mode == 0 && dense_mn && !packed && sparse_pair_left_wanted(R, Cn, dev, bn))
         return sparse_pair_left(epi, false, S_comp, meta_tiled, Dn, out, R, Cn, K, ld, tensor_scale, dev,
                                 static_cast<cudaStream_t>(stream_v));
     if (bn == 224) bn = 0;
@@ -892,7 +895,7 @@ int bm_hgemm_sparse_f32(const uint16_t* A_comp, const uint16_t* B, float* C, con
     if (int rc = current_device_state(&dev)) return rc;
     const int tiles_r = ceil_div(M, kBM);
     int bn = forced_bn();
-    if (sparse_pair_left_wanted(M, N, dev, bn, true))
+    if (sparse_pair_left_wanted(M, N, dev, bn))
         return sparse_pair_left(EPI_I32, true, A_comp, tiled, B, C, M, N, K, ldc, 1.f, dev, static_cast<cudaStream_t>(stream_v));
     // 128-column tiles: 4 stages and two accumulators fit; 256-column tiles leave room for 2 stages and
     // one accumulator only and were measured slower (4096^3: 122 vs 99 us; 8192^3: 904 vs 801 us)

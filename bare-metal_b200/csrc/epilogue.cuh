@@ -249,11 +249,17 @@ struct TmemSource {
 // NBUF staging strips per warp (1 or 2), used round-robin over the boxes of all tiles (`box_count`
 // runs on across tiles).  With two strips a box is converted while the previous one is still being
 // read by its stores — what keeps the epilogue going when the stores go to other GPUs over NVLink.
-template <int EPI, int NC, int NBUF, class Source>
+// `first_read` is called once, when the first chunk has left the accumulator; `reverse` (boxes of one chunk only) drains
+// the last chunk first.
+struct NoHook {
+    __device__ __forceinline__ void operator()() const {}
+};
+template <int EPI, int NC, int NBUF, class Source, class Hook = NoHook>
 __device__ __forceinline__ void drain_tma_from(const EpilogueParams& p, const CUtensorMap* maps, int n_maps, const Source& src,
                                                int row0, int lane, int col0, const EpiStrip<NC>* strip, float lane_s,
                                                uint32_t stage_smem0, uint32_t& box_count, int col_limit,
-                                               const StorePace& pace = StorePace{nullptr, 0u, 0u, 0}) {
+                                               const StorePace& pace = StorePace{nullptr, 0u, 0u, 0},
+                                               const Hook& first_read = Hook{}, bool reverse = false) {
     using T = typename OutType<EPI>::type;
     static_assert(NC % 32 == 0, "drained in chunks of 32 columns");
     constexpr int CHUNKS = NC / 32;
@@ -264,15 +270,19 @@ __device__ __forceinline__ void drain_tma_from(const EpilogueParams& p, const CU
     const int sw = lane & 7;                                 // 128-byte swizzle: piece index ^ (row % 8)
     uint32_t stage_smem = stage_smem0 + (NBUF > 1 ? (box_count & 1u) * kStoreBoxBytes : 0u);
 
+    auto chunk_at = [&](int i) { return CHUNKS_PER_BOX == 1 && reverse ? CHUNKS - 1 - i : i; };
+    auto live_at = [&](int i) { return col0 + chunk_at(i) * 32 < col_limit; };
     uint32_t rr[2][32];
-    if (col0 < col_limit) src.issue(0, rr[0]);
+    if (live_at(0)) src.issue(chunk_at(0), rr[0]);
 #pragma unroll
-    for (int c = 0; c < CHUNKS; ++c) {
-        const int cur = c & 1;
-        const bool live = col0 + c * 32 < col_limit;            // warp-uniform
+    for (int i = 0; i < CHUNKS; ++i) {
+        const int cur = i & 1;
+        const int c = CHUNKS_PER_BOX == 1 ? chunk_at(i) : i;
+        const bool live = live_at(i);                           // warp-uniform
+        if (live) src.wait();
+        if (i == 0) first_read();
+        if (i + 1 < CHUNKS && live_at(i + 1)) src.issue(chunk_at(i + 1), rr[cur ^ 1]);
         if (live) {
-            src.wait();
-            if (c + 1 < CHUNKS && col0 + (c + 1) * 32 < col_limit) src.issue(c + 1, rr[cur ^ 1]);
             if (c % CHUNKS_PER_BOX == 0) {
                 // the strip may still be read by the store issued NBUF boxes ago
                 stage_smem = stage_smem0 + (NBUF > 1 ? (box_count & 1u) * kStoreBoxBytes : 0u);
@@ -300,7 +310,7 @@ __device__ __forceinline__ void drain_tma_from(const EpilogueParams& p, const CU
                              : "memory");
             }
         }
-        const bool box_done = (c % CHUNKS_PER_BOX == CHUNKS_PER_BOX - 1) || c == CHUNKS - 1;
+        const bool box_done = (c % CHUNKS_PER_BOX == CHUNKS_PER_BOX - 1) || i == CHUNKS - 1;
         const int box_c0 = col0 + (c / CHUNKS_PER_BOX) * COLS_PER_BOX;
         if (box_done && box_c0 < col_limit) {
             fence_proxy_async_smem();                        // generic-proxy writes -> visible to the TMA engine

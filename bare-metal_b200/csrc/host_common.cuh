@@ -42,7 +42,7 @@ inline int fail_msg(int code, const char* what) {
 // environment variable BM_<NAME IN CAPITALS>, read ONCE when the first launcher runs, or from its
 // default; no launcher reads the environment on the launch path.  -1 means "let the launcher decide".
 enum : int {
-    OPT_FORCE_BN = 0,        // pin the tile width (0 = choose); 240 / 224 select the sparse pair kernels
+    OPT_FORCE_BN = 0,        // pin the tile width (0 = choose); 240 / 224 select the sparse pair kernels (weights / left operand)
     OPT_DENSE_PAIR,          // 0 keeps dense problems on the single-CTA kernel
     OPT_SPARSE_PAIR,         // 0 keeps sparse problems on the single-CTA kernel
     OPT_ROW_BALANCED,        // decode shapes on packed weights: rows dealt out in multiples of 8 (0 = whole tiles)

@@ -21,29 +21,36 @@ namespace bm {
 
 // LEFT = true is the reference orientation (igemm_sparse_tiled.cu:88-96, hgemm_sparse_tiled.cu:122-129):
 // the sparse operand on the left, out[r][c], the dense operand B[K x C] row-major taken as an MN-major
-// MMA operand.  A pair then computes 256 rows x 224 columns: each CTA stages ONE 128-byte-wide box of
-// B per K block at column offset 112 * rank (16-byte aligned; the MMA reads 112 of its 128 columns),
-// 52 KiB per stage and CTA, accumulators 2 x 224 + 32 metadata columns = 480.  F16 = true (LEFT only)
-// is the fp16 form: a stage covers 128 logical K, B is two boxes of 64 fp16 columns, one
-// tcgen05.cp of metadata and four tcgen05.mma.sp.kind::f16 of K = 32 (column pair + selector).
+// MMA operand.  A pair computes 256 rows x 256 columns: each CTA stages 128 columns of B per K block, 52 KiB per
+// stage and CTA.  F16 = true (LEFT only) is the fp16 form: a stage covers 128 logical K, B is two boxes of
+// 64 fp16 columns, one tcgen05.cp of metadata and four tcgen05.mma.sp.kind::f16 of K = 32 (column pair + selector).
+//
+// Why 256 columns and not the 224 or 240 that leave room for two whole accumulators: a CTA's share must start on a
+// 128-byte line.  Shares of 112 columns (or 120 fp16 columns, 240 bytes) put every 128-byte row of a B box
+// across two lines, and the fill, which bounds these kernels, dropped to ~40 B/clk/SM.
+// Two accumulators of 256 columns and the metadata do not fit 512 columns, so the accumulators OVERLAP by 32: columns
+// [0, 256) and [224, 480).  The shared columns are the last of the one and the first of the other; they are
+// drained first, and the MMAs of the next tile wait for that single chunk (`overlap` barrier) on top of the usual
+// wait for their own accumulator.
 template <bool LEFT>
 struct SpPairCfg {
-    static constexpr int BN = LEFT ? 224 : 240;
+    static constexpr int BN = LEFT ? 256 : 240;
     static constexpr int HALF_N = BN / 2;
+    static constexpr int ACC_STRIDE = LEFT ? 224 : 240;                       // columns between the two accumulators
     static constexpr int A_BYTES = 128 * 128;
-    static constexpr int B_BYTES = LEFT ? 128 * 256 : HALF_N * 256;          // 32 / 30 KiB
+    static constexpr int B_BYTES = HALF_N * 256;                              // 32 / 30 KiB
     static constexpr int STAGE_BYTES = A_BYTES + kSpMetaBytes + B_BYTES;      // 52 / 50 KiB
     // LEFT gives one ring stage to 8 x 4 KiB of store staging: its row-major fp32 / int32 output leaves
     // through TMA stores (a lane per output row makes direct stores touch 32 lines per instruction:
     // 541 us instead of 373 us for the lone-CTA kernel at 8192^3 before this)
     static constexpr int STAGES = LEFT ? 3 : 4;
-    static constexpr int E_BASE = 2 * BN;
+    static constexpr int E_BASE = ACC_STRIDE + BN;
     static constexpr int NC = 128;
     static constexpr int STORE_OFFSET = STAGES * STAGE_BYTES;
     static constexpr int BAR_OFFSET = STORE_OFFSET + (LEFT ? kEpiWarps * kStoreBoxBytes : 0);
-    static constexpr int STRIP_OFFSET = BAR_OFFSET + (2 * STAGES + 5) * 8 + 16;
+    static constexpr int STRIP_OFFSET = BAR_OFFSET + (2 * STAGES + 6) * 8 + 16;
     static constexpr int SMEM_BYTES = STRIP_OFFSET + kEpiWarps * (int)sizeof(EpiStrip<NC>) + 1024;
-    static_assert(E_BASE + STAGES * 8 <= 512, "tensor memory over-subscribed");
+    static_assert(E_BASE == 480 && STAGES * 8 <= 32, "tensor memory over-subscribed");
     static_assert(SMEM_BYTES <= 227 * 1024, "shared memory over-subscribed");
 };
 
@@ -52,7 +59,7 @@ constexpr int kSpPairBN = SpPairCfg<false>::BN;               // tokens per pair
 constexpr int kSpPairHalfN = SpPairCfg<false>::HALF_N;        // token rows staged per CTA
 constexpr int kSpPairABytes = SpPairCfg<false>::A_BYTES;      // kept values
 constexpr int kSpPairTmemCols = 512;
-constexpr int kSpPairNC = SpPairCfg<false>::NC;               // accumulator columns per epilogue warp (second half: 112 / 96 live)
+constexpr int kSpPairNC = SpPairCfg<false>::NC;               // accumulator columns per epilogue warp (second half of the sparse-weight form: 112 live)
 constexpr int kSpPairSmemBytes = SpPairCfg<false>::SMEM_BYTES;
 
 __device__ __forceinline__ void tmem_cp_128x128b_pair(uint32_t taddr, uint64_t smem_desc) {
@@ -111,9 +118,10 @@ igemm_sparse_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
     auto acc_full_bar = [&](int a) { return bar0 + 8u * (2 * kSpPairStages + a); };
     auto acc_empty_bar = [&](int a) { return bar0 + 8u * (2 * kSpPairStages + 2 + a); };
     const uint32_t drain_bar = bar0 + 8u * (2 * kSpPairStages + 4);
-    const uint32_t tmem_slot = bar0 + 8u * (2 * kSpPairStages + 5);
+    const uint32_t overlap_bar = bar0 + 8u * (2 * kSpPairStages + 5);   // LEFT, in the leader
+    const uint32_t tmem_slot = bar0 + 8u * (2 * kSpPairStages + 6);
     volatile uint32_t* tmem_slot_gen =
-        reinterpret_cast<volatile uint32_t*>(smem_gen + kSpPairBarOffset + 8 * (2 * kSpPairStages + 5));
+        reinterpret_cast<volatile uint32_t*>(smem_gen + kSpPairBarOffset + 8 * (2 * kSpPairStages + 6));
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot_gen + 1);
 
     const int warp = threadIdx.x >> 5;
@@ -135,6 +143,7 @@ igemm_sparse_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
             mbar_init(acc_empty_bar(a), 2 * kEpiWarps);
         }
         mbar_init(drain_bar, 1);
+        mbar_init(overlap_bar, kEpiWarps);               // one warp per lane quarter and CTA
         *abort_flag = 0;
         fence_mbar_init();
     }
@@ -195,12 +204,17 @@ igemm_sparse_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
         if (lane == 0 && rank == 0) {
             constexpr uint32_t idesc = F16 ? make_idesc_f16(256, kSpPairBN, true, true) : make_idesc_i8(256, kSpPairBN, LEFT, true);
             uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
+            [[maybe_unused]] uint32_t overlap_phase = 0;
             bool ok = true;
             for (int tile = pair; ok && tile < num_tiles; tile += num_pairs) {
                 if (!bounded_wait(acc_empty_bar(acc), acc_phase ^ 1u, abort_flag, p.status,
                                   DEV_TIMEOUT_MMA_ACC_EMPTY)) { ok = false; break; }
+                if (LEFT && tile != pair) {
+                    if (!bounded_wait(overlap_bar, overlap_phase, abort_flag, p.status, DEV_TIMEOUT_MMA_ACC_EMPTY)) { ok = false; break; }
+                    overlap_phase ^= 1u;
+                }
                 tc_fence_after_sync();
-                const uint32_t d_tmem = tmem_base + acc * kSpPairBN;
+                const uint32_t d_tmem = tmem_base + acc * PC::ACC_STRIDE;
                 for (int kb = 0; kb < p.k_blocks; ++kb) {
                     if (!bounded_wait(full_bar(stage), phase, abort_flag, p.status, DEV_TIMEOUT_MMA_FULL)) {
                         ok = false;
@@ -268,17 +282,28 @@ igemm_sparse_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
                 break;
             tc_fence_after_sync();
             const uint32_t taddr =
-                tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * kSpPairBN + half * kSpPairNC;
+                tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * PC::ACC_STRIDE + half * kSpPairNC;
+            // the columns both accumulators share: the last chunk of the first, the first chunk of the second one
+            [[maybe_unused]] const bool has_overlap = half != static_cast<int>(acc);
+            [[maybe_unused]] auto overlap_read = [&] {
+                if (!has_overlap) return;
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster(mapa_shared(overlap_bar, 0));
+            };
             bool stored = false;
             if constexpr (LEFT) {
                 if (p.epi.tma_ok) {
                     drain_tma_from<EPI, kSpPairNC, 1>(p.epi, &map_out, 1, TmemSource{taddr}, n0 + quarter * 32, lane, t0, strip,
                                                       lane_s, smem_base + PC::STORE_OFFSET + (warp - 2) * kStoreBoxBytes,
-                                                      box_count, t_limit);
+                                                      box_count, t_limit, StorePace{nullptr, 0u, 0u, 0}, overlap_read, half == 1);
                     stored = true;
                 }
             }
-            if (!stored) drain_accumulator<EPI, kSpPairNC, !LEFT>(p.epi, taddr, channel, t0, t_limit, strip, lane_s);
+            if (!stored) {
+                drain_accumulator<EPI, kSpPairNC, !LEFT>(p.epi, taddr, channel, t0, t_limit, strip, lane_s);
+                if constexpr (LEFT) overlap_read();
+            }
             tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(mapa_shared(acc_empty_bar(acc), 0));

@@ -58,6 +58,7 @@ __device__ __forceinline__ uint32_t lane_word(const NatWord& nat, int row, int q
 __global__ void pack_meta_rows_kernel(const uint8_t* __restrict__ rows_meta, uint8_t* __restrict__ tiled,
                                       int R, int K, int k_blocks, size_t units,
                                       MetaDest dest, int f16_lanes) {
+    pdl_launch_dependents();      // a GEMM behind this kernel may start its own set-up
     const size_t unit = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
     if (unit >= units) return;
     int row, b0;
@@ -80,6 +81,7 @@ __global__ void pack_meta_rows_kernel(const uint8_t* __restrict__ rows_meta, uin
 __global__ void pack_meta_ref_kernel(const uint32_t* __restrict__ meta_ref, uint8_t* __restrict__ tiled,
                                      int R, int K, int k_blocks, size_t units,
                                      MetaDest dest) {
+    pdl_launch_dependents();      // a GEMM behind this kernel may start its own set-up
     const size_t unit = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
     if (unit >= units) return;
     int row, b0;
@@ -103,6 +105,7 @@ __global__ void pack_meta_ref_kernel(const uint32_t* __restrict__ meta_ref, uint
 __global__ void pack_meta_ref_f16_kernel(const uint32_t* __restrict__ meta_ref, uint8_t* __restrict__ tiled,
                                          int R, int K, int k_blocks, size_t units,
                                          MetaDest dest) {
+    pdl_launch_dependents();      // a GEMM behind this kernel may start its own set-up
     const size_t unit = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
     if (unit >= units) return;
     int row, b0;

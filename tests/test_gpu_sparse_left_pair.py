@@ -1,0 +1,57 @@
+"""Sparse operand on the left on CTA pairs: several tiles per pair, so that the two accumulators, which share 32
+columns of tensor memory, are refilled while their neighbour is being drained."""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+from bare_metal_b200 import igemm as ig
+from _gpu import T, assert_clean_status, dev, forced_bn, options
+
+pytestmark = pytest.mark.gpu
+
+
+def sparse_left(M, K, seed):
+    W = oracle.gen_int8((M, K), seed, 1)
+    comp, nib = ig.prune_2_4(T(W), M, K)
+    return comp, nib, oracle.decompress_rows(comp.cpu().numpy(), nib.cpu().numpy())
+
+
+# K of one stage and less (the drain is then longer than the MMAs), of several ring turns; columns that end inside the
+# first chunk, the middle and the last chunk of a tile; rows that end inside a CTA's half
+@pytest.mark.parametrize("M,N,K", [(2304, 6160, 64), (2064, 6384, 256), (1040, 12288, 288), (2560, 4080, 1056)])
+@pytest.mark.parametrize("tma_store", [1, 0])
+def test_integers_are_exact_over_several_tiles_per_pair(M, N, K, tma_store):
+    comp, nib, dense = sparse_left(M, K, 4)
+    B = oracle.gen_int8((K, N), 4, 2)
+    tiled = ig.sp_pack_meta(nib, ig.BM_META_ROWS, M, K)
+    buf = torch.full((M + 2, N + 16), 0x5A5A5A5A, dtype=torch.int32, device=dev())
+    with options(force_bn=224, tma_store=tma_store):
+        ig.igemm_sparse_i32(comp, tiled, ig.BM_META_TILED, T(B), buf[1:M + 1, :N], M, N, K, ig.BM_B_KN)
+        assert_clean_status()
+    got = buf.cpu().numpy()
+    assert np.array_equal(got[1:M + 1, :N], oracle.igemm(dense, B, threads=0))
+    got[1:M + 1, :N] = 0x5A5A5A5A
+    assert (got == 0x5A5A5A5A).all(), "store outside the output"
+
+
+@pytest.mark.parametrize("M,N,K", [(2304, 6160, 32), (2064, 6384, 144)])
+def test_fp16_sums_of_small_integers_are_exact_over_several_tiles_per_pair(M, N, K):
+    """Integers up to 15 make every product and partial sum exact in fp32: any order gives the same bits."""
+    g = torch.Generator(device=dev()).manual_seed(3)
+    comp = torch.randint(-15, 16, (M, K // 2), device=dev(), generator=g).half()
+    B = torch.randint(-15, 16, (K, N), device=dev(), generator=g).half()
+    words = torch.full(((M // 16) * (K // 16) * 8,), 0x9CE4 | (0x9CE4 << 16), dtype=torch.int64, device=dev())
+    words = torch.where(words >= 2 ** 31, words - 2 ** 32, words).to(torch.int32)
+    out = []
+    for bn in (224, 128):
+        C = torch.full((M, N), -1.0, device=dev())
+        with forced_bn(bn):
+            ig.hgemm_sparse_tiled(comp, B, C, words, M, N, K)
+        assert_clean_status()
+        out.append(C)
+    # nibbles of a word, lowest first: 0x4 (positions 0, 1), 0xE (2, 3), 0xC (0, 3), 0x9 (1, 2)
+    pos = torch.tensor([(0, 1), (2, 3), (0, 3), (1, 2)], device=dev()).repeat(K // 16, 1)
+    cols = (torch.arange(K // 4, device=dev())[:, None] * 4 + pos).reshape(-1)
+    want = comp.double() @ B.double()[cols]
+    assert torch.equal(out[0].double(), want) and torch.equal(out[1], out[0])
