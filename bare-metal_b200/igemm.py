@@ -45,7 +45,9 @@ def _out(t: torch.Tensor, dtype, name: str) -> int:
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """Handle of the current device's current stream.  (torch.cuda.current_stream().cuda_stream is the same number by way
+    of a Stream object: 3.1 us a call against 0.2, a third of the host time of a small GEMM.)"""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 # --------------------------------------------------------------------------------------
@@ -192,8 +194,8 @@ def quantize_rows(X_f16, M, K):
     _check_f16(X_f16)
     if not X_f16.is_contiguous():
         raise BmError("X must be contiguous")
-    q = torch.empty((M, K), dtype=torch.int8, device=X_f16.device)
-    s = torch.empty(M, dtype=torch.float32, device=X_f16.device)
+    q = X_f16.new_empty((M, K), dtype=torch.int8)
+    s = X_f16.new_empty((M,), dtype=torch.float32)
     _lib.check(L.bm_quantize_rows_f16(X_f16.data_ptr(), q.data_ptr(), s.data_ptr(), M, K, _stream()),
                "bm_quantize_rows_f16")
     return q, s
