@@ -103,7 +103,7 @@ igemm_dense_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         reinterpret_cast<volatile uint32_t*>(smem_gen + Cfg::BAR_OFFSET + 8 * (2 * Cfg::STAGES + 5));
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot_gen + 1);
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0);      // known to be the same in all lanes
     const int lane = threadIdx.x & 31;
     const int num_tiles = p.tiles_m * p.tiles_n;
     constexpr uint32_t nstages = Cfg::STAGES;
@@ -134,18 +134,18 @@ igemm_dense_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
 
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer
-        if (lane == 0) {
-            prefetch_tensormap(&map_a);
-            prefetch_tensormap(&map_b);
-            uint32_t stage = 0, phase = 0, issued = 0, issued_parity = 0;
-            bool ok = true;
-            for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x) {
-                const int m0 = (tile % p.tiles_m) * kBM;
-                const int n0 = (tile / p.tiles_m) * BN;
-                for (int kb = 0; kb < p.k_blocks; ++kb) {
-                    if (!bounded_wait(empty_bar(stage), phase ^ 1u, abort_flag, p.status,
-                                      DEV_TIMEOUT_PRODUCER_EMPTY)) { ok = false; break; }
-                    const uint32_t bar = full_bar(stage);
+        prefetch_tensormap(&map_a);
+        prefetch_tensormap(&map_b);
+        uint32_t stage = 0, phase = 0, issued = 0, issued_parity = 0;
+        bool ok = true;
+        for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x) {
+            const int m0 = (tile % p.tiles_m) * kBM;
+            const int n0 = (tile / p.tiles_m) * BN;
+            for (int kb = 0; kb < p.k_blocks; ++kb) {
+                if (!warp_bounded_wait(empty_bar(stage), phase ^ 1u, abort_flag, p.status,
+                                  DEV_TIMEOUT_PRODUCER_EMPTY)) { ok = false; break; }
+                const uint32_t bar = full_bar(stage);
+                if (elect_one()) {
                     mbar_expect_tx(bar, Cfg::STAGE_BYTES);
                     tma_load_2d(a_smem0 + stage * kABytes, &map_a, bar, kb * kBK, m0);
                     if constexpr (B_MN) {
@@ -156,40 +156,41 @@ igemm_dense_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                     } else {
                         tma_load_2d(b_smem0 + stage * Cfg::B_BYTES, &map_b, bar, kb * kBK, n0);
                     }
-                    issued |= 1u << stage;
-                    issued_parity = (issued_parity & ~(1u << stage)) | (phase << stage);
-                    if (++stage == nstages) { stage = 0; phase ^= 1u; }
                 }
+                __syncwarp();
+                issued |= 1u << stage;
+                issued_parity = (issued_parity & ~(1u << stage)) | (phase << stage);
+                if (++stage == nstages) { stage = 0; phase ^= 1u; }
             }
-            if (!ok) {
-                // aborting: let the copies already in flight land before the CTA gives up its smem
-                for (int s = 0; s < Cfg::STAGES; ++s)
-                    if (issued & (1u << s)) {
-                        uint64_t t0 = global_timer_ns();
-                        while (!mbar_try_wait(full_bar(s), (issued_parity >> s) & 1u) &&
-                               global_timer_ns() - t0 < 20000000ull) {}
-                    }
-            }
+        }
+        if (!ok) {
+            // aborting: let the copies already in flight land before the CTA gives up its smem
+            for (int s = 0; s < Cfg::STAGES; ++s)
+                if (issued & (1u << s)) {
+                    uint64_t t0 = global_timer_ns();
+                    while (!mbar_try_wait(full_bar(s), (issued_parity >> s) & 1u) &&
+                           global_timer_ns() - t0 < 20000000ull) {}
+                }
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
-            constexpr uint32_t idesc = make_idesc_i8(kBM, BN, B_MN, false);
-            uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
-            bool ok = true;
-            for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x) {
-                if (!bounded_wait(acc_empty_bar(acc), acc_phase ^ 1u, abort_flag, p.status,
-                                  DEV_TIMEOUT_MMA_ACC_EMPTY)) { ok = false; break; }
+        constexpr uint32_t idesc = make_idesc_i8(kBM, BN, B_MN, false);
+        uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
+        bool ok = true;
+        for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x) {
+            if (!warp_bounded_wait(acc_empty_bar(acc), acc_phase ^ 1u, abort_flag, p.status,
+                              DEV_TIMEOUT_MMA_ACC_EMPTY)) { ok = false; break; }
+            tc_fence_after_sync();
+            const uint32_t d_tmem = tmem_base + acc * BN;
+            for (int kb = 0; kb < p.k_blocks; ++kb) {
+                if (!warp_bounded_wait(full_bar(stage), phase, abort_flag, p.status, DEV_TIMEOUT_MMA_FULL)) {
+                    ok = false;
+                    break;
+                }
                 tc_fence_after_sync();
-                const uint32_t d_tmem = tmem_base + acc * BN;
-                for (int kb = 0; kb < p.k_blocks; ++kb) {
-                    if (!bounded_wait(full_bar(stage), phase, abort_flag, p.status, DEV_TIMEOUT_MMA_FULL)) {
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after_sync();
-                    const uint32_t a_addr = a_smem0 + stage * kABytes;
-                    const uint32_t b_addr = b_smem0 + stage * Cfg::B_BYTES;
+                const uint32_t a_addr = a_smem0 + stage * kABytes;
+                const uint32_t b_addr = b_smem0 + stage * Cfg::B_BYTES;
+                if (elect_one()) {
 #pragma unroll
                     for (int ks = 0; ks < kBK / kUmmaK; ++ks) {
                         // K-major, 128B swizzle: 8-row groups are 1 KiB apart; a K step of 32 bytes
@@ -208,19 +209,22 @@ igemm_dense_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                         mma_i8(d_tmem, a_desc, b_desc, idesc, (kb | ks) != 0 ? 1u : 0u);
                     }
                     tc_commit(empty_bar(stage));            // frees the stage when these MMAs retire
-                    if (++stage == nstages) { stage = 0; phase ^= 1u; }
                 }
-                if (!ok) break;
-                tc_commit(acc_full_bar(acc));               // accumulator complete
-                acc ^= 1u;
-                if (acc == 0) acc_phase ^= 1u;
+                __syncwarp();
+                if (++stage == nstages) { stage = 0; phase ^= 1u; }
             }
-            if (!ok) {
-                // aborting: wait for MMAs in flight before tensor memory is released
-                tc_commit(drain_bar);
-                uint64_t t0 = global_timer_ns();
-                while (!mbar_try_wait(drain_bar, 0) && global_timer_ns() - t0 < 20000000ull) {}
-            }
+            if (!ok) break;
+            if (elect_one()) tc_commit(acc_full_bar(acc));   // accumulator complete
+            __syncwarp();
+            acc ^= 1u;
+            if (acc == 0) acc_phase ^= 1u;
+        }
+        if (!ok) {
+            // aborting: wait for MMAs in flight before tensor memory is released
+            if (elect_one()) tc_commit(drain_bar);
+            __syncwarp();
+            uint64_t t0 = global_timer_ns();
+            while (!mbar_try_wait(drain_bar, 0) && global_timer_ns() - t0 < 20000000ull) {}
         }
     } else {
         // ------------------------------------------------------------------ epilogue warps

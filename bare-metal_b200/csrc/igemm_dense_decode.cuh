@@ -87,7 +87,7 @@ igemm_dense_decode_kernel(const __grid_constant__ CUtensorMap map_w3, const __gr
         reinterpret_cast<volatile uint32_t*>(smem_gen + kDdBarOffset + 8 * (2 * kDdMaxStages + 7));
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot_gen + 1);
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0);      // known to be the same in all lanes
     const int lane = threadIdx.x & 31;
     const uint32_t nstages = static_cast<uint32_t>(p.stages);
     const int rot = static_cast<int>((blockIdx.x * 7u) % static_cast<unsigned>(p.k_stages));
@@ -121,77 +121,81 @@ igemm_dense_decode_kernel(const __grid_constant__ CUtensorMap map_w3, const __gr
 
     if (warp == 0 || warp == 2 + kEpiWarps) {
         // ------------------------------------------------------------------ producers: weights, activations
-        if (lane == 0) {
-            const bool is_w = warp == 0;
-            const CUtensorMap* map3 = is_w ? &map_w3 : &map_x3;
-            const CUtensorMap* map2 = is_w ? &map_w2 : &map_x2;
-            prefetch_tensormap(map3);
-            const uint32_t base = is_w ? w_smem0 : x_smem0, stage_bytes = is_w ? w_stage : x_stage;
-            const uint32_t chunk_bytes = is_w ? w_chunk : x_chunk;
-            uint32_t stage = 0, phase = 0;
-            bool ok = true;
-            for (int tile = blockIdx.x; ok && tile < p.tiles; tile += gridDim.x) {
-                const int row0 = is_w ? tile * p.tile_rows : 0;
-                for (int i = 0; i < p.k_stages; ++i) {
-                    const int ks = k_stage_of(i), c0 = ks * p.chunks;
-                    if (!bounded_wait(empty_bar(stage), phase ^ 1u, abort_flag, p.status,
-                                      DEV_TIMEOUT_PRODUCER_EMPTY)) { ok = false; break; }
-                    const uint32_t bar = full_bar(stage);
-                    const uint32_t dst = base + stage * stage_bytes;
+        const bool is_w = warp == 0;
+        const CUtensorMap* map3 = is_w ? &map_w3 : &map_x3;
+        const CUtensorMap* map2 = is_w ? &map_w2 : &map_x2;
+        prefetch_tensormap(map3);
+        const uint32_t base = is_w ? w_smem0 : x_smem0, stage_bytes = is_w ? w_stage : x_stage;
+        const uint32_t chunk_bytes = is_w ? w_chunk : x_chunk;
+        uint32_t stage = 0, phase = 0;
+        bool ok = true;
+        for (int tile = blockIdx.x; ok && tile < p.tiles; tile += gridDim.x) {
+            const int row0 = is_w ? tile * p.tile_rows : 0;
+            for (int i = 0; i < p.k_stages; ++i) {
+                const int ks = k_stage_of(i), c0 = ks * p.chunks;
+                if (!warp_bounded_wait(empty_bar(stage), phase ^ 1u, abort_flag, p.status,
+                                  DEV_TIMEOUT_PRODUCER_EMPTY)) { ok = false; break; }
+                const uint32_t bar = full_bar(stage);
+                const uint32_t dst = base + stage * stage_bytes;
+                if (elect_one()) {
                     if (is_w) mbar_expect_tx(bar, w_stage + x_stage);   // both operands
                     if (p.whole_chunks || c0 + p.chunks <= p.full_chunks) {
                         tma_load_3d(dst, map3, bar, 0, row0, c0);
                     } else {
                         for (int c = 0; c < p.chunks; ++c) tma_load_2d(dst + c * chunk_bytes, map2, bar, (c0 + c) * 128, row0);
                     }
-                    if (++stage == nstages) { stage = 0; phase ^= 1u; }
                 }
+                __syncwarp();
+                if (++stage == nstages) { stage = 0; phase ^= 1u; }
             }
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
-            const uint32_t idesc = make_idesc_i8(kBM, p.tokens_padded * p.fold, false, false);
-            const uint64_t w_desc0 = make_smem_desc(w_smem0, 0, 1024, SWIZZLE_128B_DESC);
-            const uint64_t x_desc0 = make_smem_desc(x_smem0, 0, 1024, SWIZZLE_128B_DESC);
-            uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
-            bool ok = true;
-            for (int tile = blockIdx.x; ok && tile < p.tiles; tile += gridDim.x) {
-                if (!bounded_wait(acc_empty_bar(acc), acc_phase ^ 1u, abort_flag, p.status,
-                                  DEV_TIMEOUT_MMA_ACC_EMPTY)) { ok = false; break; }
+        const uint32_t idesc = make_idesc_i8(kBM, p.tokens_padded * p.fold, false, false);
+        const uint64_t w_desc0 = make_smem_desc(w_smem0, 0, 1024, SWIZZLE_128B_DESC);
+        const uint64_t x_desc0 = make_smem_desc(x_smem0, 0, 1024, SWIZZLE_128B_DESC);
+        uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
+        bool ok = true;
+        for (int tile = blockIdx.x; ok && tile < p.tiles; tile += gridDim.x) {
+            if (!warp_bounded_wait(acc_empty_bar(acc), acc_phase ^ 1u, abort_flag, p.status,
+                              DEV_TIMEOUT_MMA_ACC_EMPTY)) { ok = false; break; }
+            tc_fence_after_sync();
+            const uint32_t d_tmem = tmem_base + acc * p.acc_stride;
+            uint32_t accumulate = 0u;
+            for (int i = 0; i < p.k_stages; ++i) {
+                if (!warp_bounded_wait(full_bar(stage), phase, abort_flag, p.status, DEV_TIMEOUT_MMA_FULL)) {
+                    ok = false;
+                    break;
+                }
                 tc_fence_after_sync();
-                const uint32_t d_tmem = tmem_base + acc * p.acc_stride;
-                uint32_t accumulate = 0u;
-                for (int i = 0; i < p.k_stages; ++i) {
-                    if (!bounded_wait(full_bar(stage), phase, abort_flag, p.status, DEV_TIMEOUT_MMA_FULL)) {
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after_sync();
+                if (elect_one()) {
                     uint64_t a_desc = w_desc0 + ((stage * w_stage) >> 4);         // addresses are in units of 16 bytes
                     uint64_t b_desc = x_desc0 + ((stage * x_stage) >> 4);
                     for (int c = 0; c < p.chunks; c += p.fold) {
 #pragma unroll
-                        for (int s = 0; s < kBK / kUmmaK; ++s) {
-                            mma_i8(d_tmem, a_desc + s * (kUmmaK >> 4), b_desc + s * (kUmmaK >> 4), idesc, accumulate);
-                            accumulate = 1u;
-                        }
+                        for (int s = 0; s < kBK / kUmmaK; ++s)
+                            mma_i8(d_tmem, a_desc + s * (kUmmaK >> 4), b_desc + s * (kUmmaK >> 4), idesc,
+                                   (c | s) != 0 ? 1u : accumulate);
                         a_desc += (w_chunk * p.fold) >> 4;
                         b_desc += (x_chunk * p.fold) >> 4;
                     }
                     tc_commit(empty_bar(stage));
-                    if (++stage == nstages) { stage = 0; phase ^= 1u; }
                 }
-                if (!ok) break;
-                tc_commit(acc_full_bar(acc));
-                acc ^= 1u;
-                if (acc == 0) acc_phase ^= 1u;
+                __syncwarp();
+                accumulate = 1u;
+                if (++stage == nstages) { stage = 0; phase ^= 1u; }
             }
-            if (!ok) {
-                tc_commit(drain_bar);
-                uint64_t t0 = global_timer_ns();
-                while (!mbar_try_wait(drain_bar, 0) && global_timer_ns() - t0 < 20000000ull) {}
-            }
+            if (!ok) break;
+            if (elect_one()) tc_commit(acc_full_bar(acc));
+            __syncwarp();
+            acc ^= 1u;
+            if (acc == 0) acc_phase ^= 1u;
+        }
+        if (!ok) {
+            if (elect_one()) tc_commit(drain_bar);
+            __syncwarp();
+            uint64_t t0 = global_timer_ns();
+            while (!mbar_try_wait(drain_bar, 0) && global_timer_ns() - t0 < 20000000ull) {}
         }
     } else {
         // ------------------------------------------------------------------ epilogue warps

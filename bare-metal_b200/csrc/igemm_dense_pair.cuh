@@ -95,7 +95,7 @@ igemm_dense_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
         reinterpret_cast<volatile uint32_t*>(smem_gen + kPairBarOffset + 8 * (2 * kPairStages + 5));
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot_gen + 1);
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0);      // known to be the same in all lanes
     const int lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();        // 0 = leader
     const uint32_t peer = rank ^ 1u;
@@ -131,25 +131,25 @@ igemm_dense_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
 
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer (both CTAs)
-        if (lane == 0) {
-            prefetch_tensormap(&map_a);
-            prefetch_tensormap(&map_b);
-            uint32_t stage = 0, phase = 0;
-            bool ok = true;
-            PairWorkIter work(pair, num_pairs, num_tiles, p.tail_first, p.tail_narrow != 0);
-            PairWork w;
-            while (ok && work.next(w)) {
-                int tm, tn;
-                pair_tile_coords(p, w.tile, tm, tn);
-                const int m0 = tm * 256 + static_cast<int>(rank) * kBM;
-                // half-height unit: 128 rows of the tile, 64 per CTA (an M = 128 pair MMA); B as for a whole tile
-                const bool narrow = w.nhalf >= 0;
-                const int n0 = tn * kPairBN + static_cast<int>(rank) * kPairHalfN;
-                const int m0s = tm * 256 + w.nhalf * 128 + static_cast<int>(rank) * 64;
-                for (int kb = 0; kb < p.k_blocks; ++kb) {
-                    if (!bounded_wait(empty_bar(stage), phase ^ 1u, abort_flag, p.status,
-                                      DEV_TIMEOUT_PRODUCER_EMPTY)) { ok = false; break; }
-                    const uint32_t leader_full = mapa_shared(full_bar(stage), 0);
+        prefetch_tensormap(&map_a);
+        prefetch_tensormap(&map_b);
+        uint32_t stage = 0, phase = 0;
+        bool ok = true;
+        PairWorkIter work(pair, num_pairs, num_tiles, p.tail_first, p.tail_narrow != 0);
+        PairWork w;
+        while (ok && work.next(w)) {
+            int tm, tn;
+            pair_tile_coords(p, w.tile, tm, tn);
+            const int m0 = tm * 256 + static_cast<int>(rank) * kBM;
+            // half-height unit: 128 rows of the tile, 64 per CTA (an M = 128 pair MMA); B as for a whole tile
+            const bool narrow = w.nhalf >= 0;
+            const int n0 = tn * kPairBN + static_cast<int>(rank) * kPairHalfN;
+            const int m0s = tm * 256 + w.nhalf * 128 + static_cast<int>(rank) * 64;
+            for (int kb = 0; kb < p.k_blocks; ++kb) {
+                if (!warp_bounded_wait(empty_bar(stage), phase ^ 1u, abort_flag, p.status,
+                                  DEV_TIMEOUT_PRODUCER_EMPTY)) { ok = false; break; }
+                const uint32_t leader_full = mapa_shared(full_bar(stage), 0);
+                if (elect_one()) {
                     if (rank == 0) mbar_expect_tx(full_bar(stage), narrow ? 2 * (kABytes / 2 + kPairBBytes) : 2 * kPairStageBytes);
                     if (narrow) tma_load_2d_pair(a_smem0 + stage * kABytes, &map_a_short, leader_full, kb * kBK, m0s);
                     else        tma_load_2d_pair(a_smem0 + stage * kABytes, &map_a, leader_full, kb * kBK, m0);
@@ -157,13 +157,14 @@ igemm_dense_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
                         tma_load_2d_pair(b_smem0 + stage * kPairBBytes, &map_b, leader_full, n0, kb * kBK);
                     else
                         tma_load_2d_pair(b_smem0 + stage * kPairBBytes, &map_b, leader_full, kb * kBK, n0);
-                    if (++stage == kPairStages) { stage = 0; phase ^= 1u; }
                 }
+                __syncwarp();
+                if (++stage == kPairStages) { stage = 0; phase ^= 1u; }
             }
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer (leader only)
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {
             constexpr uint32_t idesc_full = make_idesc_i8(256, kPairBN, B_MN, false);
             constexpr uint32_t idesc_narrow = make_idesc_i8(128, kPairBN, B_MN, false);   // 64 rows per CTA
             uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
@@ -171,39 +172,46 @@ igemm_dense_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
             PairWorkIter work(pair, num_pairs, num_tiles, p.tail_first, p.tail_narrow != 0);
             PairWork w;
             while (ok && work.next(w)) {
-                if (!bounded_wait(acc_empty_bar(acc), acc_phase ^ 1u, abort_flag, p.status,
+                if (!warp_bounded_wait(acc_empty_bar(acc), acc_phase ^ 1u, abort_flag, p.status,
                                   DEV_TIMEOUT_MMA_ACC_EMPTY)) { ok = false; break; }
                 tc_fence_after_sync();
                 const uint32_t d_tmem = tmem_base + acc * kPairBN;
                 const uint32_t idesc = w.nhalf >= 0 ? idesc_narrow : idesc_full;
                 for (int kb = 0; kb < p.k_blocks; ++kb) {
-                    if (!bounded_wait(full_bar(stage), phase, abort_flag, p.status, DEV_TIMEOUT_MMA_FULL)) {
+                    if (!warp_bounded_wait(full_bar(stage), phase, abort_flag, p.status, DEV_TIMEOUT_MMA_FULL)) {
                         ok = false;
                         break;
                     }
                     tc_fence_after_sync();
                     const uint32_t a_addr = a_smem0 + stage * kABytes;
                     const uint32_t b_addr = b_smem0 + stage * kPairBBytes;
+                    if (elect_one()) {
 #pragma unroll
-                    for (int ks = 0; ks < kBK / kUmmaK; ++ks) {
-                        const uint64_t a_desc = make_smem_desc(a_addr + ks * kUmmaK, 0, 1024, SWIZZLE_128B_DESC);
-                        const uint64_t b_desc =
-                            B_MN ? make_smem_desc(b_addr + ks * (kUmmaK * 128), 128 * kBK, 1024, SWIZZLE_128B_DESC)
-                                 : make_smem_desc(b_addr + ks * kUmmaK, 0, 1024, SWIZZLE_128B_DESC);
-                        mma_i8_pair(d_tmem, a_desc, b_desc, idesc, (kb | ks) != 0 ? 1u : 0u);
+                        for (int ks = 0; ks < kBK / kUmmaK; ++ks) {
+                            const uint64_t a_desc = make_smem_desc(a_addr + ks * kUmmaK, 0, 1024, SWIZZLE_128B_DESC);
+                            const uint64_t b_desc =
+                                B_MN ? make_smem_desc(b_addr + ks * (kUmmaK * 128), 128 * kBK, 1024, SWIZZLE_128B_DESC)
+                                     : make_smem_desc(b_addr + ks * kUmmaK, 0, 1024, SWIZZLE_128B_DESC);
+                            mma_i8_pair(d_tmem, a_desc, b_desc, idesc, (kb | ks) != 0 ? 1u : 0u);
+                        }
+                        tc_commit_pair(empty_bar(stage));                       // this CTA's producer
+                        tc_commit_pair(mapa_shared(empty_bar(stage), 1));       // the peer's producer
                     }
-                    tc_commit_pair(empty_bar(stage));                       // this CTA's producer
-                    tc_commit_pair(mapa_shared(empty_bar(stage), 1));       // the peer's producer
+                    __syncwarp();
                     if (++stage == kPairStages) { stage = 0; phase ^= 1u; }
                 }
                 if (!ok) break;
-                tc_commit_pair(acc_full_bar(acc));
-                tc_commit_pair(mapa_shared(acc_full_bar(acc), 1));
+                if (elect_one()) {
+                    tc_commit_pair(acc_full_bar(acc));
+                    tc_commit_pair(mapa_shared(acc_full_bar(acc), 1));
+                }
+                __syncwarp();
                 acc ^= 1u;
                 if (acc == 0) acc_phase ^= 1u;
             }
             if (!ok) {
-                tc_commit_pair(drain_bar);
+                if (elect_one()) tc_commit_pair(drain_bar);
+                __syncwarp();
                 uint64_t t0 = global_timer_ns();
                 while (!mbar_try_wait(drain_bar, 0) && global_timer_ns() - t0 < 20000000ull) {}
             }

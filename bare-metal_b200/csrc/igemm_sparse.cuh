@@ -169,7 +169,7 @@ igemm_sparse_kernel(const __grid_constant__ CUtensorMap map_s, const __grid_cons
         reinterpret_cast<volatile uint32_t*>(smem_gen + Cfg::BAR_OFFSET + 8 * (2 * Cfg::STAGES + 5));
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot_gen + 1);
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0);      // known to be the same in all lanes
     const int lane = threadIdx.x & 31;
     const int num_tiles = p.tiles_r * p.tiles_c;
 
@@ -199,30 +199,30 @@ igemm_sparse_kernel(const __grid_constant__ CUtensorMap map_s, const __grid_cons
 
     if (warp == 0) {
         // ------------------------------------------------------------------ producer
-        if (lane == 0) {
-            if constexpr (!PACKED) prefetch_tensormap(&map_s);
-            prefetch_tensormap(&map_d);
-            uint32_t stage = 0, phase = 0, issued = 0, issued_parity = 0;
-            bool ok = true;
-            WorkIter work(p, blockIdx.x, gridDim.x, num_tiles, ROWS);
-            WorkSegment seg;
-            while (ok && work.next(seg)) {
-                const int r0 = seg.row0;
-                const int c0 = (seg.tile / p.tiles_r) * BN;
-                // tiled metadata is laid out in 4 KiB blocks of 256 logical K; an fp16 k-block is half of one
-                const uint8_t* meta_row = p.meta_tiled + static_cast<size_t>(r0 / kBM) *
-                                                             (F16 ? (p.k_blocks + 1) / 2 : p.k_blocks) * kSpMetaBytes;
-                // packed weights: one slice of (padded rows) x 160 bytes per K block, values first
-                const size_t rows_padded = static_cast<size_t>(p.tiles_r) * kBM;
-                // Decode shapes: every CTA walks the K blocks of its tile from a different starting block and wraps
-                // around (exact integer sums do not care about the order).  All CTAs read the SAME few tokens; in
-                // lockstep they would all ask the L2 for the same 16 KiB of activations at the same moment.
-                const int rot = ROTATE_K ? static_cast<int>((blockIdx.x * 7u) % static_cast<unsigned>(p.k_blocks)) : 0;
-                for (int kb_seq = 0; kb_seq < p.k_blocks; ++kb_seq) {
-                    const int kb = kb_seq + rot < p.k_blocks ? kb_seq + rot : kb_seq + rot - p.k_blocks;
-                    if (!bounded_wait(empty_bar(stage), phase ^ 1u, abort_flag, p.status,
-                                      DEV_TIMEOUT_PRODUCER_EMPTY)) { ok = false; break; }
-                    const uint32_t bar = full_bar(stage);
+        if constexpr (!PACKED) prefetch_tensormap(&map_s);
+        prefetch_tensormap(&map_d);
+        uint32_t stage = 0, phase = 0, issued = 0, issued_parity = 0;
+        bool ok = true;
+        WorkIter work(p, blockIdx.x, gridDim.x, num_tiles, ROWS);
+        WorkSegment seg;
+        while (ok && work.next(seg)) {
+            const int r0 = seg.row0;
+            const int c0 = (seg.tile / p.tiles_r) * BN;
+            // tiled metadata is laid out in 4 KiB blocks of 256 logical K; an fp16 k-block is half of one
+            const uint8_t* meta_row = p.meta_tiled + static_cast<size_t>(r0 / kBM) *
+                                                         (F16 ? (p.k_blocks + 1) / 2 : p.k_blocks) * kSpMetaBytes;
+            // packed weights: one slice of (padded rows) x 160 bytes per K block, values first
+            const size_t rows_padded = static_cast<size_t>(p.tiles_r) * kBM;
+            // Decode shapes: every CTA walks the K blocks of its tile from a different starting block and wraps
+            // around (exact integer sums do not care about the order).  All CTAs read the SAME few tokens; in
+            // lockstep they would all ask the L2 for the same 16 KiB of activations at the same moment.
+            const int rot = ROTATE_K ? static_cast<int>((blockIdx.x * 7u) % static_cast<unsigned>(p.k_blocks)) : 0;
+            for (int kb_seq = 0; kb_seq < p.k_blocks; ++kb_seq) {
+                const int kb = kb_seq + rot < p.k_blocks ? kb_seq + rot : kb_seq + rot - p.k_blocks;
+                if (!warp_bounded_wait(empty_bar(stage), phase ^ 1u, abort_flag, p.status,
+                                  DEV_TIMEOUT_PRODUCER_EMPTY)) { ok = false; break; }
+                const uint32_t bar = full_bar(stage);
+                if (elect_one()) {
                     if constexpr (PACKED) {
                         // pre-swizzled and row-contiguous within the K block: one linear copy of the values and
                         // one of the metadata of exactly the rows of this tile (row0 is a multiple of 8, so the
@@ -254,43 +254,44 @@ igemm_sparse_kernel(const __grid_constant__ CUtensorMap map_s, const __grid_cons
                     if constexpr (!PACKED)
                         bulk_load(e_smem0 + stage * Cfg::E_BYTES, meta_row + static_cast<size_t>(kb) * kMetaStage,
                                   kMetaStage, bar);
-                    issued |= 1u << stage;
-                    issued_parity = (issued_parity & ~(1u << stage)) | (phase << stage);
-                    if (++stage == Cfg::STAGES) { stage = 0; phase ^= 1u; }
                 }
+                __syncwarp();
+                issued |= 1u << stage;
+                issued_parity = (issued_parity & ~(1u << stage)) | (phase << stage);
+                if (++stage == Cfg::STAGES) { stage = 0; phase ^= 1u; }
             }
-            if (!ok) {
-                for (int s = 0; s < Cfg::STAGES; ++s)
-                    if (issued & (1u << s)) {
-                        uint64_t t0 = global_timer_ns();
-                        while (!mbar_try_wait(full_bar(s), (issued_parity >> s) & 1u) &&
-                               global_timer_ns() - t0 < 20000000ull) {}
-                    }
-            }
+        }
+        if (!ok) {
+            for (int s = 0; s < Cfg::STAGES; ++s)
+                if (issued & (1u << s)) {
+                    uint64_t t0 = global_timer_ns();
+                    while (!mbar_try_wait(full_bar(s), (issued_parity >> s) & 1u) &&
+                           global_timer_ns() - t0 < 20000000ull) {}
+                }
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
-            constexpr uint32_t idesc = F16 ? make_idesc_f16(kBM, BN, DENSE_MN, true) : make_idesc_i8(kBM, BN, DENSE_MN, true);
-            uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
-            bool ok = true;
-            WorkIter work(p, blockIdx.x, gridDim.x, num_tiles, ROWS);
-            WorkSegment seg;
-            while (ok && work.next(seg)) {
-                if (!bounded_wait(acc_empty_bar(acc), acc_phase ^ 1u, abort_flag, p.status,
-                                  DEV_TIMEOUT_MMA_ACC_EMPTY)) { ok = false; break; }
+        constexpr uint32_t idesc = F16 ? make_idesc_f16(kBM, BN, DENSE_MN, true) : make_idesc_i8(kBM, BN, DENSE_MN, true);
+        uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
+        bool ok = true;
+        WorkIter work(p, blockIdx.x, gridDim.x, num_tiles, ROWS);
+        WorkSegment seg;
+        while (ok && work.next(seg)) {
+            if (!warp_bounded_wait(acc_empty_bar(acc), acc_phase ^ 1u, abort_flag, p.status,
+                              DEV_TIMEOUT_MMA_ACC_EMPTY)) { ok = false; break; }
+            tc_fence_after_sync();
+            const uint32_t d_tmem = tmem_base + acc * BN;
+            for (int kb = 0; kb < p.k_blocks; ++kb) {
+                if (!warp_bounded_wait(full_bar(stage), phase, abort_flag, p.status, DEV_TIMEOUT_MMA_FULL)) {
+                    ok = false;
+                    break;
+                }
                 tc_fence_after_sync();
-                const uint32_t d_tmem = tmem_base + acc * BN;
-                for (int kb = 0; kb < p.k_blocks; ++kb) {
-                    if (!bounded_wait(full_bar(stage), phase, abort_flag, p.status, DEV_TIMEOUT_MMA_FULL)) {
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after_sync();
-                    const uint32_t a_addr = a_smem0 + stage * Cfg::A_BYTES;
-                    const uint32_t b_addr = b_smem0 + stage * Cfg::B_BYTES;
-                    const uint32_t e_addr = e_smem0 + stage * Cfg::E_BYTES;
-                    const uint32_t e_tmem = tmem_base + Cfg::E_BASE + stage * 8;
+                const uint32_t a_addr = a_smem0 + stage * Cfg::A_BYTES;
+                const uint32_t b_addr = b_smem0 + stage * Cfg::B_BYTES;
+                const uint32_t e_addr = e_smem0 + stage * Cfg::E_BYTES;
+                const uint32_t e_tmem = tmem_base + Cfg::E_BASE + stage * 8;
+                if (elect_one()) {
                     // metadata: rows are 16 B apart, 8-row groups 128 B apart, no swizzle
 #pragma unroll
                     for (int j = 0; j < (F16 ? 1 : 2); ++j)
@@ -320,17 +321,20 @@ igemm_sparse_kernel(const __grid_constant__ CUtensorMap map_s, const __grid_cons
                         mma_i8_sp(d_tmem, a_desc, b_desc, e_tmem + 2 * ks, idesc, (kb != 0 || ks != 0) ? 1u : 0u);
                     }
                     tc_commit(empty_bar(stage));
-                    if (++stage == Cfg::STAGES) { stage = 0; phase ^= 1u; }
                 }
-                if (!ok) break;
-                tc_commit(acc_full_bar(acc));
-                if (++acc == Cfg::ACC_BUFS) { acc = 0; acc_phase ^= 1u; }
+                __syncwarp();
+                if (++stage == Cfg::STAGES) { stage = 0; phase ^= 1u; }
             }
-            if (!ok) {
-                tc_commit(drain_bar);
-                uint64_t t0 = global_timer_ns();
-                while (!mbar_try_wait(drain_bar, 0) && global_timer_ns() - t0 < 20000000ull) {}
-            }
+            if (!ok) break;
+            if (elect_one()) tc_commit(acc_full_bar(acc));
+            __syncwarp();
+            if (++acc == Cfg::ACC_BUFS) { acc = 0; acc_phase ^= 1u; }
+        }
+        if (!ok) {
+            if (elect_one()) tc_commit(drain_bar);
+            __syncwarp();
+            uint64_t t0 = global_timer_ns();
+            while (!mbar_try_wait(drain_bar, 0) && global_timer_ns() - t0 < 20000000ull) {}
         }
     } else {
         // ------------------------------------------------------------------ epilogue warps

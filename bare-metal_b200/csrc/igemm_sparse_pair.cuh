@@ -124,7 +124,7 @@ igemm_sparse_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
         reinterpret_cast<volatile uint32_t*>(smem_gen + kSpPairBarOffset + 8 * (2 * kSpPairStages + 6));
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot_gen + 1);
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0);      // known to be the same in all lanes
     const int lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();
     const int pair = blockIdx.x >> 1;
@@ -162,22 +162,22 @@ igemm_sparse_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
 
     if (warp == 0) {
         // ------------------------------------------------------------------ producer (both CTAs)
-        if (lane == 0) {
-            prefetch_tensormap(&map_w);
-            prefetch_tensormap(&map_e);
-            prefetch_tensormap(&map_x);
-            uint32_t stage = 0, phase = 0;
-            bool ok = true;
-            for (int tile = pair; ok && tile < num_tiles; tile += num_pairs) {
-                const int rb = tile_rb(tile) * 2 + static_cast<int>(rank);       // 128-row block of the sparse operand
-                const int t0 = tile_cb(tile) * kSpPairBN + static_cast<int>(rank) * kSpPairHalfN;
-                // metadata chunks of 128 rows x 16 B (= 128 logical K): 2 per int8 K block, 1 per fp16 K block;
-                // a row block holds 2 * ceil(K / 256) of them
-                const int chunks_per_rb = F16 ? ((p.k_blocks + 1) / 2) * 2 : p.k_blocks * 2;
-                for (int kb = 0; kb < p.k_blocks; ++kb) {
-                    if (!bounded_wait(empty_bar(stage), phase ^ 1u, abort_flag, p.status,
-                                      DEV_TIMEOUT_PRODUCER_EMPTY)) { ok = false; break; }
-                    const uint32_t leader_full = mapa_shared(full_bar(stage), 0);
+        prefetch_tensormap(&map_w);
+        prefetch_tensormap(&map_e);
+        prefetch_tensormap(&map_x);
+        uint32_t stage = 0, phase = 0;
+        bool ok = true;
+        for (int tile = pair; ok && tile < num_tiles; tile += num_pairs) {
+            const int rb = tile_rb(tile) * 2 + static_cast<int>(rank);       // 128-row block of the sparse operand
+            const int t0 = tile_cb(tile) * kSpPairBN + static_cast<int>(rank) * kSpPairHalfN;
+            // metadata chunks of 128 rows x 16 B (= 128 logical K): 2 per int8 K block, 1 per fp16 K block;
+            // a row block holds 2 * ceil(K / 256) of them
+            const int chunks_per_rb = F16 ? ((p.k_blocks + 1) / 2) * 2 : p.k_blocks * 2;
+            for (int kb = 0; kb < p.k_blocks; ++kb) {
+                if (!warp_bounded_wait(empty_bar(stage), phase ^ 1u, abort_flag, p.status,
+                                  DEV_TIMEOUT_PRODUCER_EMPTY)) { ok = false; break; }
+                const uint32_t leader_full = mapa_shared(full_bar(stage), 0);
+                if (elect_one()) {
                     if (rank == 0) mbar_expect_tx(full_bar(stage), 2 * kStageTx);
                     tma_load_2d_pair(a_smem0 + stage * kSpPairABytes, &map_w, leader_full, kb * 128, rb * 128);
                     tma_load_2d_pair(e_smem0 + stage * kSpMetaBytes, &map_e, leader_full, 0,
@@ -195,28 +195,29 @@ igemm_sparse_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
                             tma_load_2d_pair(b_addr + j * (kSpPairHalfN * 128), &map_x, leader_full,
                                              kb * kSpKLogical + j * 128, t0);
                     }
-                    if (++stage == kSpPairStages) { stage = 0; phase ^= 1u; }
                 }
+                __syncwarp();
+                if (++stage == kSpPairStages) { stage = 0; phase ^= 1u; }
             }
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer (leader only)
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {
             constexpr uint32_t idesc = F16 ? make_idesc_f16(256, kSpPairBN, true, true) : make_idesc_i8(256, kSpPairBN, LEFT, true);
             uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
             [[maybe_unused]] uint32_t overlap_phase = 0;
             bool ok = true;
             for (int tile = pair; ok && tile < num_tiles; tile += num_pairs) {
-                if (!bounded_wait(acc_empty_bar(acc), acc_phase ^ 1u, abort_flag, p.status,
+                if (!warp_bounded_wait(acc_empty_bar(acc), acc_phase ^ 1u, abort_flag, p.status,
                                   DEV_TIMEOUT_MMA_ACC_EMPTY)) { ok = false; break; }
                 if (LEFT && tile != pair) {
-                    if (!bounded_wait(overlap_bar, overlap_phase, abort_flag, p.status, DEV_TIMEOUT_MMA_ACC_EMPTY)) { ok = false; break; }
+                    if (!warp_bounded_wait(overlap_bar, overlap_phase, abort_flag, p.status, DEV_TIMEOUT_MMA_ACC_EMPTY)) { ok = false; break; }
                     overlap_phase ^= 1u;
                 }
                 tc_fence_after_sync();
                 const uint32_t d_tmem = tmem_base + acc * PC::ACC_STRIDE;
                 for (int kb = 0; kb < p.k_blocks; ++kb) {
-                    if (!bounded_wait(full_bar(stage), phase, abort_flag, p.status, DEV_TIMEOUT_MMA_FULL)) {
+                    if (!warp_bounded_wait(full_bar(stage), phase, abort_flag, p.status, DEV_TIMEOUT_MMA_FULL)) {
                         ok = false;
                         break;
                     }
@@ -225,39 +226,46 @@ igemm_sparse_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
                     const uint32_t b_addr = b_smem0 + stage * kSpPairBBytes;
                     const uint32_t e_addr = e_smem0 + stage * kSpMetaBytes;
                     const uint32_t e_tmem = tmem_base + kSpPairEBase + stage * 8;
+                    if (elect_one()) {
 #pragma unroll
-                    for (int j = 0; j < (F16 ? 1 : 2); ++j)
-                        tmem_cp_128x128b_pair(e_tmem + 4 * j, make_smem_desc(e_addr + j * 2048, 0, 128, SWIZZLE_NONE_DESC));
+                        for (int j = 0; j < (F16 ? 1 : 2); ++j)
+                            tmem_cp_128x128b_pair(e_tmem + 4 * j, make_smem_desc(e_addr + j * 2048, 0, 128, SWIZZLE_NONE_DESC));
 #pragma unroll
-                    for (int ks = 0; ks < 4; ++ks) {
-                        const uint64_t a_desc = make_smem_desc(a_addr + ks * 32, 0, 1024, SWIZZLE_128B_DESC);
-                        if constexpr (F16) {
-                            // 32 K rows per MMA; the second 64-column group is one box (128 x 128 B) further
-                            const uint64_t b_desc = make_smem_desc(b_addr + ks * (32 * 128), 128 * 128, 1024, SWIZZLE_128B_DESC);
-                            mma_f16_sp_pair(d_tmem, a_desc, b_desc, e_tmem + (ks & ~1), idesc | static_cast<uint32_t>(ks & 1),
-                                            (kb | ks) != 0 ? 1u : 0u);
-                        } else if constexpr (LEFT) {
-                            // 64 K rows of 128 B per MMA, a single 128-column group per CTA
-                            const uint64_t b_desc = make_smem_desc(b_addr + ks * (64 * 128), 128 * kKRows, 1024, SWIZZLE_128B_DESC);
-                            mma_i8_sp_pair(d_tmem, a_desc, b_desc, e_tmem + 2 * ks, idesc, (kb | ks) != 0 ? 1u : 0u);
-                        } else {
-                            const uint64_t b_desc = make_smem_desc(b_addr + (ks >> 1) * (kSpPairHalfN * 128) + (ks & 1) * 64,
-                                                                   0, 1024, SWIZZLE_128B_DESC);
-                            mma_i8_sp_pair(d_tmem, a_desc, b_desc, e_tmem + 2 * ks, idesc, (kb | ks) != 0 ? 1u : 0u);
+                        for (int ks = 0; ks < 4; ++ks) {
+                            const uint64_t a_desc = make_smem_desc(a_addr + ks * 32, 0, 1024, SWIZZLE_128B_DESC);
+                            if constexpr (F16) {
+                                // 32 K rows per MMA; the second 64-column group is one box (128 x 128 B) further
+                                const uint64_t b_desc = make_smem_desc(b_addr + ks * (32 * 128), 128 * 128, 1024, SWIZZLE_128B_DESC);
+                                mma_f16_sp_pair(d_tmem, a_desc, b_desc, e_tmem + (ks & ~1), idesc | static_cast<uint32_t>(ks & 1),
+                                                (kb | ks) != 0 ? 1u : 0u);
+                            } else if constexpr (LEFT) {
+                                // 64 K rows of 128 B per MMA, a single 128-column group per CTA
+                                const uint64_t b_desc = make_smem_desc(b_addr + ks * (64 * 128), 128 * kKRows, 1024, SWIZZLE_128B_DESC);
+                                mma_i8_sp_pair(d_tmem, a_desc, b_desc, e_tmem + 2 * ks, idesc, (kb | ks) != 0 ? 1u : 0u);
+                            } else {
+                                const uint64_t b_desc = make_smem_desc(b_addr + (ks >> 1) * (kSpPairHalfN * 128) + (ks & 1) * 64,
+                                                                       0, 1024, SWIZZLE_128B_DESC);
+                                mma_i8_sp_pair(d_tmem, a_desc, b_desc, e_tmem + 2 * ks, idesc, (kb | ks) != 0 ? 1u : 0u);
+                            }
                         }
+                        tc_commit_pair(empty_bar(stage));
+                        tc_commit_pair(mapa_shared(empty_bar(stage), 1));
                     }
-                    tc_commit_pair(empty_bar(stage));
-                    tc_commit_pair(mapa_shared(empty_bar(stage), 1));
+                    __syncwarp();
                     if (++stage == kSpPairStages) { stage = 0; phase ^= 1u; }
                 }
                 if (!ok) break;
-                tc_commit_pair(acc_full_bar(acc));
-                tc_commit_pair(mapa_shared(acc_full_bar(acc), 1));
+                if (elect_one()) {
+                    tc_commit_pair(acc_full_bar(acc));
+                    tc_commit_pair(mapa_shared(acc_full_bar(acc), 1));
+                }
+                __syncwarp();
                 acc ^= 1u;
                 if (acc == 0) acc_phase ^= 1u;
             }
             if (!ok) {
-                tc_commit_pair(drain_bar);
+                if (elect_one()) tc_commit_pair(drain_bar);
+                __syncwarp();
                 uint64_t t0 = global_timer_ns();
                 while (!mbar_try_wait(drain_bar, 0) && global_timer_ns() - t0 < 20000000ull) {}
             }

@@ -44,6 +44,11 @@ __device__ __forceinline__ uint64_t global_timer_ns() {
     return t;
 }
 
+// One lane of a warp that is here as a whole.  Copies and MMAs are issued under this, in code that the whole warp runs
+// through, never by "if (lane == 0)": their operands are warp-uniform, and from a branch that looks divergent each of
+// them costs its lane extra instructions.  Measured with the operands resident, commits and waits included:
+// tcgen05.mma i8 128 x 128 107 clocks an instruction from a lane-0 branch and 64 from an elected lane (the tensor
+// pipe's own time), CTA pair 256 x 128 122 and 64, sparse pair 256 x 240 152 and 120, sparse 128 x 16 137 and 56.
 __device__ __forceinline__ bool elect_one() {
     uint32_t pred;
     asm volatile(
@@ -129,6 +134,12 @@ __device__ __forceinline__ bool bounded_wait(uint32_t bar, uint32_t parity, vola
             }
         }
     }
+}
+
+// The same by a whole warp, with one answer for all of its lanes.
+__device__ __forceinline__ bool warp_bounded_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
+                                                  int* status, int code) {
+    return __all_sync(0xFFFFFFFFu, bounded_wait(bar, parity, abort_flag, status, code));
 }
 
 // ----------------------------------------------------------------------------------------
