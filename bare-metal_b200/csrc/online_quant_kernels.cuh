@@ -15,23 +15,37 @@
 #include <cstdint>
 #include <cuda_fp16.h>
 
+#include "sm100_ptx.cuh"
+
 namespace bm {
 
 constexpr int kOqRowBlock = 128;
 constexpr int kOqKTile = 32;
 
 // One launch does both steps.  A CTA owns a chunk of 32768 elements inside ONE scale block — 128 rows x
-// 256 columns of A, or 256 (128) rows x 128 (256) columns of B — first takes the block's maximum over
-// the first K tile itself (4096 / 8192 elements, an L2 hit for all but the first CTA of a block), then
-// converts its chunk: 16 elements per thread and step, two 16-byte loads, one 16-byte store.  The CTAs
-// of chunk 0 also publish the dequantisation scale max / 127 per row / column for the GEMM epilogue.
+// 256 columns of A, or 256 (128) rows x 128 (256) columns of B.  It asks for its whole chunk first, 64 elements a
+// thread in registers, then takes the block's maximum over the first K tile itself (4096 / 8192 elements, an
+// L2 hit for all but the first CTA of a block) while those loads are under way, and converts: two
+// 16-byte loads and one 16-byte store per 16 elements.  The CTAs of chunk 0 also publish the dequantisation scale
+// max / 127 per row / column for the GEMM epilogue.
 // K % 16 == 0 and N % 16 == 0, so a 16-element unit never straddles an edge.
+// Bound by HBM: 3 bytes per element (the GEMM behind it takes the rest of the time at the larger sizes).  With both steps,
+// before (256 threads, loads after the maximum, conversions of ~14 instructions an element) -> now: 256^3 10.2 ->
+// 7.7 us, 512 x 512 x 4096 15.7 -> 13.3, 8192 x 512 x 512 14.8 -> 12.5, 8192 x 4096 x 1024 58.7 -> 52.6, 4096^3 74.0 -> 72.7.
 constexpr int kOqChunkElems = 32768;
-constexpr int kOqThreads = 256;
+constexpr int kOqThreads = 512;
+constexpr int kOqUnits = kOqChunkElems / 16 / kOqThreads;      // 16-element units a thread holds
 
-__device__ __forceinline__ float oq_unit_max(const __half* p) {
-    const uint4 lo = reinterpret_cast<const uint4*>(p)[0], hi = reinterpret_cast<const uint4*>(p)[1];
-    const uint32_t in[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+struct OqUnit {
+    uint4 lo, hi;
+};
+
+__device__ __forceinline__ OqUnit oq_load(const __half* p) {
+    return {__ldg(reinterpret_cast<const uint4*>(p)), __ldg(reinterpret_cast<const uint4*>(p) + 1)};
+}
+
+__device__ __forceinline__ float oq_unit_max(const OqUnit& u) {
+    const uint32_t in[8] = {u.lo.x, u.lo.y, u.lo.z, u.lo.w, u.hi.x, u.hi.y, u.hi.z, u.hi.w};
     float m = 0.f;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -41,46 +55,80 @@ __device__ __forceinline__ float oq_unit_max(const __half* p) {
     return m;
 }
 
-__device__ __forceinline__ void oq_unit_convert(const __half* src, int8_t* dst, float inv) {
-    const uint4 lo = reinterpret_cast<const uint4*>(src)[0], hi = reinterpret_cast<const uint4*>(src)[1];
-    const uint32_t in[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-    uint32_t out[4] = {0, 0, 0, 0};
+// q = clamp(rint(x * inv), -128, 127), NaN -> 0.  Rounding by adding 1.5 * 2^23: the sum's low byte is the integer,
+// ties to even like rint; values beyond the type are clamped before, in a form that keeps NaNs, and a NaN shows in
+// a bit that no sum has (a unit that holds one takes the conversions instead).
+__device__ __forceinline__ uint4 oq_unit_convert(const OqUnit& u, float inv) {
+    const uint32_t in[8] = {u.lo.x, u.lo.y, u.lo.z, u.lo.w, u.hi.x, u.hi.y, u.hi.z, u.hi.w};
+    constexpr float kMagic = 12582912.f;
+    uint32_t out[4], seen = 0;
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
-        const __half h = __ushort_as_half(static_cast<unsigned short>((in[j >> 1] >> (16 * (j & 1))) & 0xFFFFu));
-        int q = __float2int_rn(__fmul_rn(__half2float(h), inv));
-        q = max(-128, min(127, q));
-        out[j >> 2] |= (static_cast<uint32_t>(q) & 0xFFu) << (8 * (j & 3));
+    for (int g = 0; g < 4; ++g) {
+        uint32_t z[4];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&in[2 * g + j]));
+            const float y0 = __fmul_rn(f.x, inv), y1 = __fmul_rn(f.y, inv);
+            float c0, c1;
+            asm("max.NaN.f32 %0, %1, 0fC3000000;" : "=f"(c0) : "f"(y0));          // -128
+            asm("max.NaN.f32 %0, %1, 0fC3000000;" : "=f"(c1) : "f"(y1));
+            asm("min.NaN.f32 %0, %1, 0f42FE0000;" : "=f"(c0) : "f"(c0));          // 127
+            asm("min.NaN.f32 %0, %1, 0f42FE0000;" : "=f"(c1) : "f"(c1));
+            z[2 * j] = __float_as_uint(__fadd_rn(c0, kMagic));
+            z[2 * j + 1] = __float_as_uint(__fadd_rn(c1, kMagic));
+        }
+        seen |= z[0] | z[1] | z[2] | z[3];
+        out[g] = __byte_perm(__byte_perm(z[0], z[1], 0x0040), __byte_perm(z[2], z[3], 0x0040), 0x5410);
     }
-    *reinterpret_cast<uint4*>(dst) = make_uint4(out[0], out[1], out[2], out[3]);
+    if (seen & 0x10000000u) {                    // sums are 0x4B3FFF80 .. 0x4B40007F, a NaN is 0x7F......
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            const __half h = __ushort_as_half(static_cast<unsigned short>((in[j >> 1] >> (16 * (j & 1))) & 0xFFFFu));
+            const int q = max(-128, min(127, __float2int_rn(__fmul_rn(__half2float(h), inv))));
+            out[j >> 2] = (out[j >> 2] & ~(0xFFu << (8 * (j & 3)))) | (static_cast<uint32_t>(q) & 0xFFu) << (8 * (j & 3));
+        }
+    }
+    return make_uint4(out[0], out[1], out[2], out[3]);
 }
 
-__global__ void __launch_bounds__(kOqThreads)
+__global__ void __launch_bounds__(kOqThreads, 2)
 oq_quantize_kernel(const __half* __restrict__ A, const __half* __restrict__ B, int8_t* __restrict__ Aq,
                    int8_t* __restrict__ Bq, float* __restrict__ row_scale, float* __restrict__ col_scale, int M, int N,
                    int K, int col_block, int chunks_a, int a_chunks_per_block, int b_chunks_per_block) {
     __shared__ float warp_max[kOqThreads / 32];
+    pdl_launch_dependents();      // the GEMM behind this kernel may start its own set-up
     const int kt = K < kOqKTile ? K : kOqKTile;
     const int tid = threadIdx.x;
     const bool is_a = static_cast<int>(blockIdx.x) < chunks_a;
     const int id = is_a ? blockIdx.x : blockIdx.x - chunks_a;
     const int per = is_a ? a_chunks_per_block : b_chunks_per_block;
     const int blk = id / per, chunk = id % per;
-    // operand-independent view: `rows` x `cols` matrix with pitch `pitch`, the chunk at (r0, c0) is
-    // ch_rows x ch_cols, the first-K-tile window at (w_r0, w_c0) is w_rows x w_cols
+    // operand-independent view: `rows` x `cols` matrix, the chunk at (r0, c0) is ch_rows x 2^units_log units of 16
+    // columns, the first-K-tile window at (w_r0, w_c0) is w_rows x w_cols
     const __half* X = is_a ? A : B;
     int8_t* Xq = is_a ? Aq : Bq;
     const int rows = is_a ? M : K, cols = is_a ? K : N;
-    const int ch_cols = is_a ? 256 : col_block, ch_rows = kOqChunkElems / ch_cols;
-    const int r0 = is_a ? blk * kOqRowBlock : chunk * ch_rows, c0 = is_a ? chunk * ch_cols : blk * col_block;
+    const int units_log = is_a || col_block == 256 ? 4 : 3;
+    const int ch_rows = (kOqChunkElems / 16) >> units_log;
+    const int r0 = is_a ? blk * kOqRowBlock : chunk * ch_rows, c0 = is_a ? chunk * 256 : blk * col_block;
     const int w_r0 = is_a ? r0 : 0, w_c0 = is_a ? 0 : c0;
     const int w_rows = is_a ? kOqRowBlock : kt, w_cols = is_a ? kt : col_block;
-    const int w_units_per_row = (w_cols + 15) / 16;
 
+    // a thread's units lie below one another, `step` rows apart
+    const int first_r = r0 + (tid >> units_log), my_c = c0 + (tid & ((1 << units_log) - 1)) * 16;
+    const int step = kOqThreads >> units_log;
+    const int mine = my_c < cols ? rows - first_r : 0;     // unit i exists if i * step < mine
+    const size_t at = static_cast<size_t>(first_r) * cols + my_c, pitch = static_cast<size_t>(step) * cols;
+    OqUnit held[kOqUnits];
+#pragma unroll
+    for (int i = 0; i < kOqUnits; ++i)
+        if (i * step < mine) held[i] = oq_load(X + at + i * pitch);
+
+    const int w_log = is_a ? 1 : units_log;               // window units per row: 2 (of which K < 32 has one) or those of the chunk
     float m = 0.f;
-    for (int u = tid; u < w_rows * w_units_per_row; u += kOqThreads) {
-        const int r = w_r0 + u / w_units_per_row, c = w_c0 + (u % w_units_per_row) * 16;
-        if (r < rows && c < cols && c < w_c0 + w_cols) m = fmaxf(m, oq_unit_max(X + static_cast<size_t>(r) * cols + c));
+    for (int u = tid; u < w_rows << w_log; u += kOqThreads) {
+        const int r = w_r0 + (u >> w_log), c = w_c0 + (u & ((1 << w_log) - 1)) * 16;
+        if (r < rows && c < cols && c < w_c0 + w_cols) m = fmaxf(m, oq_unit_max(oq_load(X + static_cast<size_t>(r) * cols + c)));
     }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, off));
@@ -97,15 +145,9 @@ oq_quantize_kernel(const __half* __restrict__ A, const __half* __restrict__ B, i
         for (int i = tid; i < count; i += kOqThreads)
             if (first + i < limit) dst[first + i] = scale;
     }
-    const int units_per_row = ch_cols / 16;
-#pragma unroll 4
-    for (int u = tid; u < kOqChunkElems / 16; u += kOqThreads) {
-        const int r = r0 + u / units_per_row, c = c0 + (u % units_per_row) * 16;
-        if (r < rows && c < cols) {
-            const size_t e = static_cast<size_t>(r) * cols + c;
-            oq_unit_convert(X + e, Xq + e, inv);
-        }
-    }
+#pragma unroll
+    for (int i = 0; i < kOqUnits; ++i)
+        if (i * step < mine) *reinterpret_cast<uint4*>(Xq + at + i * pitch) = oq_unit_convert(held[i], inv);
 }
 
 }  // namespace bm
