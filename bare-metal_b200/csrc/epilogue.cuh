@@ -339,4 +339,48 @@ __device__ __forceinline__ void drain_accumulator_tma(const EpilogueParams& p, c
                                   box_count, col_limit, pace);
 }
 
+// Drain of 128 accumulator columns of 4-byte results through boxes of 32 rows x 16 columns (64 bytes): half the staging of
+// drain_tma_from, for the kernel that needs the rest for a ring stage.  `reverse` starts at the last box;
+// `two_read` is called once, when the first two boxes (32 columns) have left the accumulator.  No column-side parameters.
+constexpr int kNarrowBoxCols = 16;
+constexpr int kNarrowBoxBytes = 32 * kNarrowBoxCols * 4;          // 2 KiB per warp
+template <int EPI, class Hook>
+__device__ __forceinline__ void drain_narrow_boxes(const EpilogueParams& p, const CUtensorMap* map, uint32_t taddr, int row0, int lane,
+                                                   int col0, uint32_t stage_smem, int col_limit, bool reverse, const Hook& two_read) {
+    static_assert(EPI == EPI_I32 || EPI == EPI_F32_TENSOR, "4-byte results without column parameters");
+    constexpr int BOXES = 128 / kNarrowBoxCols;
+    auto box_at = [&](int i) { return reverse ? BOXES - 1 - i : i; };
+    auto live_at = [&](int i) { return col0 + box_at(i) * kNarrowBoxCols < col_limit; };      // warp-uniform
+    uint32_t rr[2][16];
+    if (live_at(0)) tmem_ld_32x16(taddr + box_at(0) * kNarrowBoxCols, rr[0]);
+#pragma unroll
+    for (int i = 0; i < BOXES; ++i) {
+        if (live_at(i)) tmem_ld_wait();
+        if (i == 1) two_read();
+        if (i + 1 < BOXES && live_at(i + 1)) tmem_ld_32x16(taddr + box_at(i + 1) * kNarrowBoxCols, rr[(i + 1) & 1]);
+        if (!live_at(i)) continue;
+        if (lane == 0) bulk_wait_read_all();                     // the box before this one has been fetched
+        __syncwarp();
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+            uint32_t o[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const auto c = convert_acc<EPI>(static_cast<int32_t>(rr[i & 1][4 * v + j]), p.tensor_scale, 0.f, 0.f, 0);
+                o[j] = *reinterpret_cast<const uint32_t*>(&c);
+            }
+            // 64-byte swizzle: 16-byte piece ^ (row / 2) % 4
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(stage_smem + lane * 64 + ((v ^ ((lane >> 1) & 3)) << 4)),
+                         "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3])
+                         : "memory");
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+            tma_store_2d(map, stage_smem, col0 + box_at(i) * kNarrowBoxCols, row0);
+            bulk_commit_group();
+        }
+    }
+}
+
 }  // namespace bm

@@ -214,12 +214,12 @@ inline MapCache& map_cache() {
 // Encodes (or fetches) a tiled map of rank 2 or 3.  dims / box are innermost first; `pitch` is the byte
 // stride of dimension 1; dimension 2 of a rank-3 map steps by 128 bytes (K blocks of a row-major operand).
 inline int cached_tensor_map(CUtensorMap* map, const void* base, int rank, CUtensorMapDataType type, int elem_size,
-                             const uint64_t (&dims)[3], uint64_t pitch, const uint32_t (&box)[3], bool swizzle128,
-                             bool l2_promote) {
+                             const uint64_t (&dims)[3], uint64_t pitch, const uint32_t (&box)[3],
+                             CUtensorMapSwizzle swizzle, bool l2_promote) {
     EncodeTiledFn fn = encode_tiled_fn();
     if (!fn) return fail_msg(BM_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
     MapKey key{base, dims[0], dims[1], rank == 3 ? dims[2] : 0, pitch, box[0], box[1], rank == 3 ? box[2] : 0,
-               static_cast<uint32_t>(elem_size) | (swizzle128 ? 1u << 8 : 0u) | (static_cast<uint32_t>(rank) << 16) |
+               static_cast<uint32_t>(elem_size) | (static_cast<uint32_t>(swizzle) << 8) | (static_cast<uint32_t>(rank) << 16) |
                    (l2_promote ? 1u << 24 : 0u)};
     MapCache& cache = map_cache();
     {
@@ -236,7 +236,7 @@ inline int cached_tensor_map(CUtensorMap* map, const void* base, int rank, CUten
     cuuint32_t gbox[3] = {box[0], box[1], box[2]};
     cuuint32_t elem_strides[3] = {1, 1, 1};
     CUresult r = fn(map, type, static_cast<cuuint32_t>(rank), const_cast<void*>(base), gdims, strides, gbox, elem_strides,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
                     l2_promote ? CU_TENSOR_MAP_L2_PROMOTION_L2_256B : CU_TENSOR_MAP_L2_PROMOTION_NONE,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) {
@@ -256,7 +256,8 @@ inline int make_tensor_map_u8(CUtensorMap* map, const void* base, uint64_t cols,
                               uint64_t pitch, uint32_t box_cols, uint32_t box_rows, bool swizzle128) {
     const uint64_t dims[3] = {cols, rows, 1};
     const uint32_t box[3] = {box_cols, box_rows, 1};
-    return cached_tensor_map(map, base, 2, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, dims, pitch, box, swizzle128, true);
+    return cached_tensor_map(map, base, 2, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, dims, pitch, box,
+                             swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, true);
 }
 
 // K-major byte matrix [rows x K] seen as [k_blocks][rows][128 bytes]: one box holds `box_blocks` K blocks of box_rows
@@ -265,17 +266,18 @@ inline int make_tensor_map_kblocks(CUtensorMap* map, const void* base, uint64_t 
                                    uint32_t box_rows, uint32_t box_blocks) {
     const uint64_t dims[3] = {128, rows, k_blocks};
     const uint32_t box[3] = {128, box_rows, box_blocks};
-    return cached_tensor_map(map, base, 3, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, dims, pitch, box, true, true);
+    return cached_tensor_map(map, base, 3, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, dims, pitch, box, CU_TENSOR_MAP_SWIZZLE_128B, true);
 }
 
-// Output matrix [rows x cols] of 2- or 4-byte elements for TMA stores: box = 128 bytes x 32 rows,
-// 128-byte swizzle (matches the staging strips of the epilogue); stores are clipped to the extent.
+// Output matrix [rows x cols] of 2- or 4-byte elements for TMA stores: box = 128 (or 64) bytes x 32 rows with the swizzle
+// of that width (matches the staging strips of the epilogue); stores are clipped to the extent.
 inline int make_tensor_map_out(CUtensorMap* map, const void* base, uint64_t cols, uint64_t rows,
-                               uint64_t pitch_bytes, int elem_size) {
+                               uint64_t pitch_bytes, int elem_size, int box_bytes = 128) {
     const uint64_t dims[3] = {cols, rows, 1};
-    const uint32_t box[3] = {static_cast<uint32_t>(128 / elem_size), 32, 1};
+    const uint32_t box[3] = {static_cast<uint32_t>(box_bytes / elem_size), 32, 1};
     return cached_tensor_map(map, base, 2, elem_size == 2 ? CU_TENSOR_MAP_DATA_TYPE_UINT16 : CU_TENSOR_MAP_DATA_TYPE_UINT32,
-                             elem_size, dims, pitch_bytes, box, true, false);
+                             elem_size, dims, pitch_bytes, box,
+                             box_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, false);
 }
 
 // Launch with programmatic stream serialization (and optionally a 2-CTA cluster): the kernel may be

@@ -32,7 +32,7 @@ namespace bm {
 // [0, 256) and [224, 480).  The shared columns are the last of the one and the first of the other; they are
 // drained first, and the MMAs of the next tile wait for that single chunk (`overlap` barrier) on top of the usual
 // wait for their own accumulator.
-template <bool LEFT>
+template <bool LEFT, int STAGES_ = 4>
 struct SpPairCfg {
     static constexpr int BN = LEFT ? 256 : 240;
     static constexpr int HALF_N = BN / 2;
@@ -40,16 +40,18 @@ struct SpPairCfg {
     static constexpr int A_BYTES = 128 * 128;
     static constexpr int B_BYTES = HALF_N * 256;                              // 32 / 30 KiB
     static constexpr int STAGE_BYTES = A_BYTES + kSpMetaBytes + B_BYTES;      // 52 / 50 KiB
-    // LEFT gives one ring stage to 8 x 4 KiB of store staging: its row-major fp32 / int32 output leaves
-    // through TMA stores (a lane per output row makes direct stores touch 32 lines per instruction:
-    // 541 us instead of 373 us for the lone-CTA kernel at 8192^3 before this)
-    static constexpr int STAGES = LEFT ? 3 : 4;
+    // LEFT stores its row-major fp32 / int32 output through TMA (a lane per output row makes direct stores touch 32 lines
+    // per instruction: 541 us instead of 373 us for the lone-CTA kernel at 8192^3).  With three ring stages a warp
+    // stages boxes of 32 columns, 4 KiB; with four (there are no strips of column parameters in this orientation) boxes of
+    // 16 columns, which drain slower: the launcher takes four for fp16 and from three waves up.
+    static constexpr int STAGES = STAGES_;
+    static constexpr bool NARROW = LEFT && STAGES == 4;
     static constexpr int E_BASE = ACC_STRIDE + BN;
     static constexpr int NC = 128;
     static constexpr int STORE_OFFSET = STAGES * STAGE_BYTES;
-    static constexpr int BAR_OFFSET = STORE_OFFSET + (LEFT ? kEpiWarps * kStoreBoxBytes : 0);
+    static constexpr int BAR_OFFSET = STORE_OFFSET + (LEFT ? kEpiWarps * (NARROW ? kNarrowBoxBytes : kStoreBoxBytes) : 0);
     static constexpr int STRIP_OFFSET = BAR_OFFSET + (2 * STAGES + 6) * 8 + 16;
-    static constexpr int SMEM_BYTES = STRIP_OFFSET + kEpiWarps * (int)sizeof(EpiStrip<NC>) + 1024;
+    static constexpr int SMEM_BYTES = STRIP_OFFSET + (LEFT ? 0 : kEpiWarps * (int)sizeof(EpiStrip<NC>)) + 1024;
     static_assert(E_BASE == 480 && STAGES * 8 <= 32, "tensor memory over-subscribed");
     static_assert(SMEM_BYTES <= 227 * 1024, "shared memory over-subscribed");
 };
@@ -91,12 +93,12 @@ __device__ __forceinline__ void mma_f16_sp_pair(uint32_t d_tmem, uint64_t a_desc
 
 // map_w: kept values (byte map); map_e: tiled metadata as rows of 128 B = 8 units (box: 32 rows, 16 for fp16);
 // map_x: the dense operand — tokens [M x K] (K-major), or B[K x C] as a byte map when LEFT
-template <int EPI, bool LEFT = false, bool F16 = false>
+template <int EPI, bool LEFT = false, bool F16 = false, int STAGES_ = 4>
 __global__ void __launch_bounds__(kDenseThreads, 1)
 igemm_sparse_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_e,
                          const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_out,
                          const SparseParams p) {
-    using PC = SpPairCfg<LEFT>;
+    using PC = SpPairCfg<LEFT, STAGES_>;
     constexpr int kSpPairStages = PC::STAGES;
     static_assert(!F16 || (LEFT && EPI == EPI_I32), "fp16: reference orientation, accumulator bits stored as they are");
     constexpr int kSpPairBN = PC::BN, kSpPairHalfN = PC::HALF_N, kSpPairBBytes = PC::B_BYTES;
@@ -302,9 +304,14 @@ igemm_sparse_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
             bool stored = false;
             if constexpr (LEFT) {
                 if (p.epi.tma_ok) {
-                    drain_tma_from<EPI, kSpPairNC, 1>(p.epi, &map_out, 1, TmemSource{taddr}, n0 + quarter * 32, lane, t0, strip,
-                                                      lane_s, smem_base + PC::STORE_OFFSET + (warp - 2) * kStoreBoxBytes,
-                                                      box_count, t_limit, StorePace{nullptr, 0u, 0u, 0}, overlap_read, half == 1);
+                    if constexpr (PC::NARROW)
+                        drain_narrow_boxes<EPI>(p.epi, &map_out, taddr, n0 + quarter * 32, lane, t0,
+                                                smem_base + PC::STORE_OFFSET + (warp - 2) * kNarrowBoxBytes, t_limit,
+                                                half == 1, overlap_read);
+                    else
+                        drain_tma_from<EPI, kSpPairNC, 1>(p.epi, &map_out, 1, TmemSource{taddr}, n0 + quarter * 32, lane, t0, strip,
+                                                          lane_s, smem_base + PC::STORE_OFFSET + (warp - 2) * kStoreBoxBytes,
+                                                          box_count, t_limit, StorePace{nullptr, 0u, 0u, 0}, overlap_read, half == 1);
                     stored = true;
                 }
             }

@@ -19,7 +19,7 @@ def sparse_left(M, K, seed):
 
 # K of one stage and less (the drain is then longer than the MMAs), of several ring turns; columns that end inside the
 # first chunk, the middle and the last chunk of a tile; rows that end inside a CTA's half
-@pytest.mark.parametrize("M,N,K", [(2304, 6160, 64), (2064, 6384, 256), (1040, 12288, 288), (2560, 4080, 1056)])
+@pytest.mark.parametrize("M,N,K", [(2304, 6160, 64), (2064, 6384, 256), (1040, 12288, 288), (2560, 4080, 1056), (1040, 6160, 320)])
 @pytest.mark.parametrize("tma_store", [1, 0])
 def test_integers_are_exact_over_several_tiles_per_pair(M, N, K, tma_store):
     comp, nib, dense = sparse_left(M, K, 4)
