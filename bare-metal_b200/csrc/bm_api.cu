@@ -79,9 +79,9 @@ struct DenseDecodePlan {
     float us;
 };
 // The fewest tiles per SM that fit, and the fold that needs the least tensor time.  `us` is a fit to W8A8 fp16-output
-// runs with 1 to 256 tokens over weights from 512 x 4096 to 28672 x 8192 (within ~20 %): launch, ramp and drain 3.6 us; the
-// weights at 5.9 TB/s or the MMAs (57 clocks each at least, half a clock per column from 114 columns up); on top the
-// activations, which every tile reads again out of L2, at 80 KB/us and SM, and the drain of the tokens.
+// runs with 1 to 256 tokens over weights from 512 x 4096 to 28672 x 8192 (within ~15 %): launch, ramp and drain 3.2 us; the
+// longest of the weights at 6.8 TB/s, one SM's share of both operands at 105 KB/us, and the MMAs (57 clocks each at
+// least, half a clock per column from 114 columns up); the drain of the tokens.
 static DenseDecodePlan plan_dense_decode(int M, int N, int K, int sms) {
     const int bn = (M + 15) / 16 * 16, k_chunks = ceil_div(K, kBK);
     const int groups = ceil_div(N, 8);                                           // channels in groups of 8
@@ -95,8 +95,10 @@ static DenseDecodePlan plan_dense_decode(int M, int N, int K, int sms) {
                          (bn * fold < 114 ? 57.f : bn * fold / 2.f) / 1.8e3f;
         if (fold == 1 || us < mma) { mma = us; plan.fold = fold; }
     }
-    const float hbm = static_cast<float>(N) * K / 5.9e6f;
-    plan.us = 3.6f + (hbm > mma ? hbm : mma) + (M > 16 ? static_cast<float>(waves) * bn * K / 80e3f + 0.02f * M : 0.f);
+    const float hbm = static_cast<float>(N) * K / 6.8e6f, fill = static_cast<float>(waves) * (rows + bn) * K / 105e3f;
+    float body = hbm > fill ? hbm : fill;
+    if (mma > body) body = mma;
+    plan.us = 3.2f + body + 0.008f * M;
     return plan;
 }
 
@@ -131,14 +133,19 @@ static int dense_decode(int epi, const int8_t* X, const int8_t* W, const Epilogu
     if (p.stages > kDdMaxStages) p.stages = kDdMaxStages;
     p.k_stages = ceil_div(k_chunks, p.chunks);
     p.status = dev->status;
-    CUtensorMap w2, x2, w3, x3;
-    if (int rc = make_tensor_map_u8(&w2, W, K, N, K, kBK, p.tile_rows, true)) return rc;
-    if (int rc = make_tensor_map_u8(&x2, X, K, M, K, kBK, p.tokens_padded, true)) return rc;
-    w3 = w2;
-    x3 = x2;
-    if (p.whole_chunks || p.full_chunks >= p.chunks) {            // else every stage takes the 2-D maps
+    CUtensorMap w2, x2, w3, x3;                                  // a pair that no stage takes is a copy of the other
+    const bool any3 = p.whole_chunks || p.full_chunks >= p.chunks;
+    if (any3) {
         if (int rc = make_tensor_map_kblocks(&w3, W, p.full_chunks, N, K, p.tile_rows, p.chunks)) return rc;
         if (int rc = make_tensor_map_kblocks(&x3, X, p.full_chunks, M, K, p.tokens_padded, p.chunks)) return rc;
+    }
+    if (!p.whole_chunks) {                                       // a ragged last K block
+        if (int rc = make_tensor_map_u8(&w2, W, K, N, K, kBK, p.tile_rows, true)) return rc;
+        if (int rc = make_tensor_map_u8(&x2, X, K, M, K, kBK, p.tokens_padded, true)) return rc;
+        if (!any3) { w3 = w2; x3 = x2; }
+    } else {
+        w2 = w3;
+        x2 = x3;
     }
     const int grid = p.tiles < dev->sm_count ? p.tiles : dev->sm_count;
     switch (epi) {
@@ -187,9 +194,11 @@ static int dense_gemm(int epi, const int8_t* A, const int8_t* B, void* C, int M,
         // The per-wave figures (us at K = 4096, W8A8 fp16 out, one B200) were measured on problems from
         // 64 x 512 to 4352 x 8192: narrow tiles move more operand bytes per MAC but finish a wave sooner,
         // so they win while the wide tiles would leave SMs idle, and lose once they need a second wave.
-        struct Cand { int bn; bool pair; float wave_us, start_us; };
-        const Cand cands[4] = {{256, true, 12.0f, 3.6f}, {256, false, 12.3f, 3.0f}, {128, false, 9.8f, 2.8f},
-                               {64, false, 9.3f, 2.6f}};
+        // (The order of the candidates was measured with these; few_wave / few_start say what one of them takes by itself
+        // with few tokens, for the comparison with the channels-on-lanes kernel below.)
+        struct Cand { int bn; bool pair; float wave_us, start_us, few_wave, few_start; };
+        const Cand cands[4] = {{256, true, 12.0f, 3.6f, 12.0f, 3.4f}, {256, false, 12.3f, 3.0f, 13.5f, 2.8f},
+                               {128, false, 9.8f, 2.8f, 7.8f, 2.6f}, {64, false, 9.3f, 2.6f, 6.0f, 2.4f}};
         const int min_bn = (b_mn || n_peers > 0) ? 128 : 64;
         float best = 0.f;
         bool best_pair = false;
@@ -200,19 +209,20 @@ static int dense_gemm(int epi, const int8_t* A, const int8_t* B, void* C, int M,
             const float cost = c.start_us + static_cast<float>((tiles + slots - 1) / slots) * c.wave_us;
             if (bn == 0 || cost < best) {
                 best = cost; bn = c.bn; best_pair = c.pair;
-                tile_us = c.start_us + (cost - c.start_us) * (K / 4096.f);
+                tile_us = c.few_start + static_cast<float>((tiles + slots - 1) / slots) * c.few_wave * (K / 4096.f);
             }
         }
         pair_ok = best_pair;
     }
-    // Few tokens on weights [N x K]: channels on the lanes.  Up to 16 tokens always (the wide tiles spend 11 to 36 us
-    // on zero-filled token rows: 4096 x 4096, 16 tokens 14.4 -> 7.0 us; 12288 x 4096 20.3 -> 12.6; 22016 x 4096
-    // 32.0 -> 22.2; 4096 x 11008 25.0 -> 12.1), above that where the model sees it ahead (4096 x 11008, 32 tokens 25.1 -> 12.3
-    // and 96 tokens 25.4 -> 20.7; but 12288 x 4096, 64 tokens 13.3 against 14.9, and 1024 x 1024 4.3 against 5.5).  The wide
-    // tiles cannot beat the weights' own streaming time either: 22016 x 4096, 32 tokens 21.4 us for 1 wave of 12.3.
+    // Few tokens on weights [N x K]: channels on the lanes.  Up to 16 tokens always (the wide tiles spend 3 to 30 us on
+    // zero-filled token rows; 16 tokens, wide -> lanes: 4096 x 4096 14.3 -> 5.9 us, 12288 x 4096 21.4 -> 10.2, 22016 x 4096 32.7 ->
+    // 16.2, 4096 x 11008 18.7 -> 9.9, 28672 x 8192 41.6 -> 36.5), above that where the model sees it ahead (12288 x 4096, 96
+    // tokens 12.7 -> 11.0; 4096 x 11008, 64 tokens 18.8 -> 13.3; but 128 tokens 19.2 against 21.5, and 1024 x 1024, 64
+    // tokens 3.6 against 4.6).  The wide tiles also stream the weights more slowly than their own model says: 22016 x 4096,
+    // 32 tokens 20.9 us for one wave.
     if (!b_mn && n_peers == 0 && M <= kDdMaxTokens && epi != EPI_F32_ROWCOL && opt(OPT_DENSE_DECODE) != 0) {
         const DenseDecodePlan plan = plan_dense_decode(M, N, K, dev->sm_count);
-        const float stream_us = 2.6f + 1.15f * N * K / 5.9e6f;
+        const float stream_us = 2.8f + 1.35f * N * K / 6.8e6f;
         const float wide_us = tile_us > stream_us ? tile_us : stream_us;
         if (opt(OPT_DENSE_DECODE) == 1 || (!bn_forced && (M <= 16 || plan.us < wide_us)))
             return dense_decode(epi, A, B, p.epi, M, N, K, plan, dev, static_cast<cudaStream_t>(stream_v));

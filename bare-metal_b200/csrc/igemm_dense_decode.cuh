@@ -18,15 +18,14 @@
 // sums, exact integers, through shared memory.
 //
 // A ring stage covers `chunks` K blocks of 128 bytes, a multiple of `fold`.  W and X are described to the TMA as [K / 128][rows][128 B],
-// so one copy fetches all chunks of an operand's stage — a copy instruction costs its thread ~140 clocks,
-// and a 32-row box of one chunk is only 4 KiB.  The last, ragged chunk of a K that is not a multiple of
+// so one copy fetches all chunks of an operand's stage: a 32-row box of one chunk is only 4 KiB.  The last, ragged chunk of a K that is not a multiple of
 // 128 comes through a plain 2-D map instead, which zero-fills beyond K.  All stage geometry is a launch
 // parameter: one instantiation per epilogue.
 //
-// What bounds it: the weights' stream from HBM plus ~3.6 us of launch, ramp and drain for one wave; the round trips of
-// the ring where tokens take most of it (64 tokens and more).  16 tokens, before (wide tiles) -> without folding ->
-// now: 4096 x 4096 14.4 -> 10.3 -> 7.0 us, 4096 x 11008 25.0 -> 22.4 -> 12.1, 8192 x 8192 19.7 -> 20.1 -> 16.4,
-// 12288 x 4096 20.3 -> 12.5 -> 12.6 (no fold: 88 channels a tile), 512 x 4096 10.1 -> 8.3 -> 4.7.
+// What bounds it: the weights' stream from HBM (28672 x 8192, 1 token: 35.5 us = 6.6 TB/s) plus ~3.2 us of launch, ramp and
+// drain; with many tokens what one SM can take in of both operands.  16 tokens, before (wide tiles) -> without folding ->
+// folded -> with copies and MMAs from an elected lane: 4096 x 4096 14.4 -> 10.3 -> 7.0 -> 5.9 us, 4096 x 11008 25.0 -> 22.4 ->
+// 12.1 -> 9.9, 12288 x 4096 20.3 -> 12.5 -> 12.6 (88 channels a tile: no fold) -> 10.2, 512 x 4096 10.1 -> 8.3 -> 4.7 -> 3.9.
 //
 // Every CTA starts its K walk at another stage and wraps around (exact integer sums do not depend on the
 // order), so the CTAs do not ask the L2 for the same activations at the same moment.
