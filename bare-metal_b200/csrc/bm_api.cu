@@ -460,18 +460,19 @@ static int sparse_pair_left(int epi, bool f16, const void* S_comp, const uint8_t
     return fail_msg(BM_ERR_LAYOUT, "unsupported epilogue for the sparse pair kernel");
 }
 
-// When the reference orientation runs on CTA pairs (256 x 256 tiles) instead of lone CTAs (128 x 128): by waves.  One wave of
-// pair tiles takes about 1.4 lone ones (per 4096 of K: int8 11.1 against 7.9 us, fp16 16.8 against 12.4), so
-// pairs win wherever they need fewer than 5/7 of the waves.  Lone CTAs -> pairs: 2048 x 2048 x 2048 (2 waves against 1) int8
-// 14.9 -> 12.0 us, fp16 18.2 -> 12.2; 2048 x 4096 x 4096 (4, 2) 35.7 -> 26.1, 53.7 -> 37.6; 8192^3 (28, 14) 441 -> 313,
-// 890 -> 602; but 1024 x 2048 x 4096 (1, 1) 13.7 -> 14.5, 16.4 -> 16.8.  Tile width 224 forces pairs.
+// When the reference orientation runs on CTA pairs (256 x 256 tiles) instead of lone CTAs (128 x 128): where they need
+// fewer waves.  Lone CTAs -> pairs (waves) over 26 shapes of ragged and even sizes: 1.3 to 1.9 times faster wherever pairs
+// need fewer (5408 x 1616 x 1600 (4, 3) int8 31.0 -> 24.3 us, fp16 33.8 -> 25.9; 2528 x 1536 x 7648 (2, 1) 32.6 -> 19.9, 45.1 -> 27.4;
+// 5904 x 6736 x 768 (17, 9) 106 -> 54, 104 -> 54), and within 3 % of one another, either way, where both need the same
+// (1600 x 1200 x 6752 (1, 1) 26.6 -> 27.4, 28.0 -> 26.9; 4912 x 832 x 2560 (2, 2) 16.6 -> 16.9, 19.2 -> 19.1).  Tile width 224
+// forces pairs.
 static bool sparse_pair_left_wanted(int R, int Cn, const DeviceState* dev, int forced) {
     if (forced == 224) return dev->sm_count >= 2;
     if (forced != 0 || dev->sm_count < 2 || opt(OPT_SPARSE_PAIR) == 0) return false;
     auto waves = [&](int rows, int cols, int slots) {
         return (static_cast<long long>(ceil_div(R, rows)) * ceil_div(Cn, cols) + slots - 1) / slots;
     };
-    return 7 * waves(256, SpPairCfg<true>::BN, dev->sm_count / 2) < 5 * waves(128, 128, dev->sm_count);
+    return waves(256, SpPairCfg<true>::BN, dev->sm_count / 2) < waves(128, 128, dev->sm_count);
 }
 
 // option "sparse_pair" = 0 keeps large sparse-weight problems on the single-CTA kernel (testing hook)
