@@ -17,9 +17,10 @@
 // partial sums of `fold` K ranges (the other blocks are never read).  The epilogue adds the `fold` partial
 // sums, exact integers, through shared memory.
 //
-// A ring stage covers `chunks` K blocks of 128 bytes, a multiple of `fold`.  W and X are described to the TMA as [K / 128][rows][128 B],
-// so one copy fetches all chunks of an operand's stage: a 32-row box of one chunk is only 4 KiB.  The last, ragged chunk of a K that is not a multiple of
-// 128 comes through a plain 2-D map instead, which zero-fills beyond K.  All stage geometry is a launch
+// A ring stage covers `chunks` K blocks of 128 bytes, a multiple of `fold`.  W and X are described to the TMA as
+// [K / 128][rows][128 B], so one copy fetches all chunks of an operand's stage: a 32-row box of one chunk is only
+// 4 KiB.  The last, ragged chunk of a K that is not a multiple of 128 comes through a plain 2-D map instead, which
+// zero-fills beyond K (chunks that do not exist arrive as zeros either way).  All stage geometry is a launch
 // parameter: one instantiation per epilogue.
 //
 // What bounds it: the weights' stream from HBM (28672 x 8192, 1 token: 35.5 us = 6.6 TB/s) plus ~3.2 us of launch, ramp and
