@@ -46,8 +46,12 @@ def _out(t: torch.Tensor, dtype, name: str) -> int:
 
 def _stream() -> int:
     """Handle of the current device's current stream.  (torch.cuda.current_stream().cuda_stream is the same number by way
-    of a Stream object: 3.1 us a call against 0.2, a third of the host time of a small GEMM.)"""
-    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    of a Stream object: 3.1 us a call against 0.2, a third of the host time of a small GEMM.  The raw calls are private to
+    torch: without them the object it is.)"""
+    try:
+        return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    except AttributeError:
+        return torch.cuda.current_stream().cuda_stream
 
 
 # --------------------------------------------------------------------------------------

@@ -118,3 +118,22 @@ def test_gather_and_barrier_entry_points_reject_bad_arguments_without_a_device()
     assert L.bm_peer_barrier(None, 2, 0, None) == -1
     assert L.bm_peer_barrier(ptrs, 2, 2, None) == -2
     assert L.bm_peer_barrier(ptrs, 9, 0, None) == -1
+
+
+def test_stream_handle_without_the_private_torch_calls(monkeypatch):
+    """torch's raw-handle calls are private names: where one is missing, the public stream object gives the handle."""
+    import torch
+    from bare_metal_b200 import igemm
+
+    class Stream:
+        cuda_stream = 0x51
+
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda *a: Stream)
+    monkeypatch.setattr(torch._C, "_cuda_getDevice", lambda: 3, raising=False)
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda d: 0x70 + d, raising=False)
+    assert igemm._stream() == 0x73
+    monkeypatch.delattr(torch._C, "_cuda_getCurrentRawStream")
+    assert igemm._stream() == 0x51
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda d: 0x70 + d, raising=False)
+    monkeypatch.delattr(torch._C, "_cuda_getDevice")
+    assert igemm._stream() == 0x51
