@@ -198,8 +198,11 @@ def quantize_rows(X_f16, M, K):
     _check_f16(X_f16)
     if not X_f16.is_contiguous():
         raise BmError("X must be contiguous")
-    q = X_f16.new_empty((M, K), dtype=torch.int8)
-    s = X_f16.new_empty((M,), dtype=torch.float32)
+    if type(X_f16) is torch.Tensor:                  # 1.6 us an allocation against 2.3, but a subclass would get its own type
+        q, s = X_f16.new_empty((M, K), dtype=torch.int8), X_f16.new_empty((M,), dtype=torch.float32)
+    else:
+        q = torch.empty((M, K), dtype=torch.int8, device=X_f16.device)
+        s = torch.empty(M, dtype=torch.float32, device=X_f16.device)
     _lib.check(L.bm_quantize_rows_f16(X_f16.data_ptr(), q.data_ptr(), s.data_ptr(), M, K, _stream()),
                "bm_quantize_rows_f16")
     return q, s

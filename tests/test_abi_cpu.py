@@ -137,3 +137,26 @@ def test_stream_handle_without_the_private_torch_calls(monkeypatch):
     monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda d: 0x70 + d, raising=False)
     monkeypatch.delattr(torch._C, "_cuda_getDevice")
     assert igemm._stream() == 0x51
+
+
+def test_quantiser_returns_plain_tensors_for_a_tensor_subclass(monkeypatch):
+    import torch
+    from bare_metal_b200 import igemm
+
+    class Tagged(torch.Tensor):
+        pass
+
+    class Library:
+        @staticmethod
+        def bm_quantize_rows_f16(*args):
+            return 0
+
+    monkeypatch.setattr(igemm, "_check_f16", lambda t: True)
+    monkeypatch.setattr(igemm, "_stream", lambda: 0)
+    monkeypatch.setattr(igemm._lib, "load", lambda: Library)
+    x = torch.zeros((3, 16), dtype=torch.float16)
+    for arg in (x, x.as_subclass(Tagged), torch.nn.Parameter(x)):
+        q, s = igemm.quantize_rows(arg, 3, 16)
+        assert type(q) is torch.Tensor and type(s) is torch.Tensor
+        assert (q.shape, q.dtype, s.shape, s.dtype) == ((3, 16), torch.int8, (3,), torch.float32)
+        assert not q.requires_grad and not s.requires_grad
