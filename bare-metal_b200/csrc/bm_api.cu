@@ -90,7 +90,8 @@ static DenseDecodePlan plan_dense_decode(int M, int N, int K, int sms) {
     DenseDecodePlan plan{rows, 1, 0.f};
     float mma = 0.f;
     for (int fold = 1; fold <= 8; fold *= 2) {
-        if (fold > 1 && (rows * fold > kBM || bn * fold > 256 || rows * fold * bn > kDdPartInts || fold > k_chunks)) break;
+        // the folded epilogue is written for a CTA's only tile (tiles of a second wave have 72 channels or more and do not fit)
+        if (fold > 1 && (waves > 1 || rows * fold > kBM || bn * fold > 256 || rows * fold * bn > kDdPartInts || fold > k_chunks)) break;
         const float us = static_cast<float>(waves) * ceil_div(k_chunks, fold) * 4.f *
                          (bn * fold < 114 ? 57.f : bn * fold / 2.f) / 1.8e3f;
         if (fold == 1 || us < mma) { mma = us; plan.fold = fold; }

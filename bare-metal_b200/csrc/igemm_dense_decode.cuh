@@ -15,7 +15,8 @@
 // matrix of chunk * h rows; `fold` chunks of W stacked on the 128 lanes against `fold` chunks of X stacked on
 // the columns are ONE MMA whose diagonal blocks — channels of chunk i against tokens of chunk i — are the
 // partial sums of `fold` K ranges (the other blocks are never read).  The epilogue adds the `fold` partial
-// sums, exact integers, through shared memory.
+// sums, exact integers, through shared memory.  A folded CTA has one tile: more than one tile per SM means tiles of 72
+// channels or more, which do not fold.
 //
 // A ring stage covers `chunks` K blocks of 128 bytes, a multiple of `fold`.  W and X are described to the TMA as
 // [K / 128][rows][128 B], so one copy fetches all chunks of an operand's stage: a 32-row box of one chunk is only
@@ -43,7 +44,7 @@ constexpr int kDdRingBytes = 176 * 1024;
 constexpr int kDdPartInts = 8192;                         // partial sums of a folded tile: fold * h * padded tokens
 constexpr int kDdThreads = 96 + 32 * kEpiWarps;           // W producer, MMA issuer, epilogue warps, X producer
 constexpr int kDdBarOffset = kDdRingBytes;
-constexpr int kDdStripOffset = kDdBarOffset + (2 * kDdMaxStages + 7) * 8 + 24;
+constexpr int kDdStripOffset = kDdBarOffset + (2 * kDdMaxStages + 6) * 8 + 24;
 constexpr int kDdPartOffset = (kDdStripOffset + kEpiWarps * kDdMaxTokens * 4 + 127) / 128 * 128;
 constexpr int kDdSmemBytes = kDdPartOffset + kDdPartInts * 4 + 1024;
 static_assert(kDdSmemBytes <= 227 * 1024, "shared memory over-subscribed");
@@ -52,10 +53,10 @@ struct DenseDecodeParams {
     EpilogueParams epi;                // out [rows = tokens x cols = channels]
     int tiles, tile_rows;              // channels per tile (h)
     int tokens_padded;                 // accumulator columns in use: tokens rounded up to 16
-    int fold;                          // K blocks side by side in one MMA (1: none)
+    int fold;                          // K blocks side by side in one MMA (1: none); above 1 only with tiles <= grid
     int acc_stride, tmem_cols;         // columns between the two accumulators; columns allocated
     int chunks, stages;                // K blocks of 128 bytes per ring stage; ring stages
-    int full_chunks, whole_chunks;     // K blocks entirely inside K; there are no others (and at least one stage of them)
+    int full_chunks, whole_chunks;     // K blocks entirely inside K; 1: there are no others (K % 128 == 0)
     int k_stages;                      // stages that cover K
     int* status;
 };
@@ -80,11 +81,10 @@ igemm_dense_decode_kernel(const __grid_constant__ CUtensorMap map_w3, const __gr
     auto acc_full_bar = [&](int a) { return bar0 + 8u * (2 * kDdMaxStages + a); };
     auto acc_empty_bar = [&](int a) { return bar0 + 8u * (2 * kDdMaxStages + 2 + a); };
     const uint32_t drain_bar = bar0 + 8u * (2 * kDdMaxStages + 4);
-    const uint32_t parked_bar = bar0 + 8u * (2 * kDdMaxStages + 5);   // folded tiles: partial sums written / read
-    const uint32_t added_bar = bar0 + 8u * (2 * kDdMaxStages + 6);
-    const uint32_t tmem_slot = bar0 + 8u * (2 * kDdMaxStages + 7);
+    const uint32_t parked_bar = bar0 + 8u * (2 * kDdMaxStages + 5);   // folded tile: partial sums written
+    const uint32_t tmem_slot = bar0 + 8u * (2 * kDdMaxStages + 6);
     volatile uint32_t* tmem_slot_gen =
-        reinterpret_cast<volatile uint32_t*>(smem_gen + kDdBarOffset + 8 * (2 * kDdMaxStages + 7));
+        reinterpret_cast<volatile uint32_t*>(smem_gen + kDdBarOffset + 8 * (2 * kDdMaxStages + 6));
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot_gen + 1);
 
     const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0);      // known to be the same in all lanes
@@ -104,7 +104,6 @@ igemm_dense_decode_kernel(const __grid_constant__ CUtensorMap map_w3, const __gr
         }
         mbar_init(drain_bar, 1);
         mbar_init(parked_bar, kEpiWarps);
-        mbar_init(added_bar, kEpiWarps);
         *abort_flag = 0;
         fence_mbar_init();
     }
@@ -209,7 +208,7 @@ igemm_dense_decode_kernel(const __grid_constant__ CUtensorMap map_w3, const __gr
             for (int t = lane; t < tokens; t += 32) strip[t] = __ldg(p.epi.row_scale + t);
             __syncwarp();
         }
-        uint32_t acc = 0, acc_phase = 0, fold_phase = 0;
+        uint32_t acc = 0, acc_phase = 0;
         for (int tile = blockIdx.x; tile < p.tiles; tile += gridDim.x) {
             const int in_tile = quarter * 32 + lane;
             const int channel = tile * p.tile_rows + in_tile;
@@ -239,13 +238,9 @@ igemm_dense_decode_kernel(const __grid_constant__ CUtensorMap map_w3, const __gr
                         }
                     }
                 }
-                tc_fence_before_sync();
                 __syncwarp();
-                if (lane == 0) {
-                    mbar_arrive(acc_empty_bar(acc));
-                    mbar_arrive(parked_bar);
-                }
-                if (!bounded_wait(parked_bar, fold_phase, abort_flag, p.status, DEV_TIMEOUT_EPI_ACC_FULL)) break;
+                if (lane == 0) mbar_arrive(parked_bar);
+                if (!bounded_wait(parked_bar, 0, abort_flag, p.status, DEV_TIMEOUT_EPI_ACC_FULL)) break;
                 const int part = p.tokens_padded * p.tile_rows;
                 for (int c = lane; c < p.tile_rows; c += 32) {
                     const int ch = tile * p.tile_rows + c;
@@ -262,14 +257,7 @@ igemm_dense_decode_kernel(const __grid_constant__ CUtensorMap map_w3, const __gr
                             convert_acc<EPI>(sum, p.epi.tensor_scale, s, EPI == EPI_F16_ROWCOL ? strip[t] : s, z);
                     }
                 }
-                // the next tile parks in the same place
-                __syncwarp();
-                if (lane == 0) mbar_arrive(added_bar);
-                if (!bounded_wait(added_bar, fold_phase, abort_flag, p.status, DEV_TIMEOUT_EPI_ACC_FULL)) break;
-                fold_phase ^= 1u;
-                acc ^= 1u;
-                if (acc == 0) acc_phase ^= 1u;
-                continue;
+                break;                                       // the CTA's only tile
             }
             if (quarter * 32 < p.tile_rows) {                                    // warp-uniform
                 const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * p.acc_stride;
