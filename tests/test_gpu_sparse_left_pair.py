@@ -55,3 +55,33 @@ def test_fp16_sums_of_small_integers_are_exact_over_several_tiles_per_pair(M, N,
     cols = (torch.arange(K // 4, device=dev())[:, None] * 4 + pos).reshape(-1)
     want = comp.double() @ B.double()[cols]
     assert torch.equal(out[0].double(), want) and torch.equal(out[1], out[0])
+
+
+# the borders of a 256 x 256 tile and of a CTA's 128 columns and rows, and one 16-column step to either side
+@pytest.mark.parametrize("M,N", [(256, 256), (240, 240), (272, 272), (512, 128), (144, 512), (400, 496), (1024, 2304)])
+def test_tile_borders(M, N):
+    K = 544
+    comp, nib, dense = sparse_left(M, K, 9)
+    B = oracle.gen_int8((K, N), 9, 2)
+    tiled = ig.sp_pack_meta(nib, ig.BM_META_ROWS, M, K)
+    C = torch.full((M, N), -1, dtype=torch.int32, device=dev())
+    with options(force_bn=224):
+        ig.igemm_sparse_i32(comp, tiled, ig.BM_META_TILED, T(B), C, M, N, K, ig.BM_B_KN)
+        assert_clean_status()
+    assert np.array_equal(C.cpu().numpy(), oracle.igemm(dense, B, threads=0))
+
+
+# the launcher's own choice behind the reference ABI: 225 pair tiles on 74 pairs (four ring stages, stores in boxes of 16
+# columns), 108 (three stages, boxes of 32), few enough for lone CTAs
+@pytest.mark.parametrize("M,N,K", [(2064, 6384, 64), (2064, 6384, 320), (2304, 2832, 96), (1040, 1040, 96)])
+def test_scaled_fp32_results_where_the_launcher_chooses(M, N, K):
+    dense = oracle.gen_sparse_2_4_ref(M, K, 5)
+    comp, meta = oracle.compress_2_4_ref(dense)
+    B = oracle.gen_int8((K, N), 5, 2)
+    buf = torch.full((M + 2, N), -1.0, device=dev())
+    ig.igemm_sparse_tiled(T(comp), T(B), buf[1:M + 1], T(meta.view(np.int32)), M, N, K, 0.011, 0.007)
+    assert_clean_status()
+    got = buf.cpu().numpy()
+    assert (got[0] == -1).all() and (got[-1] == -1).all(), "store outside the output"
+    want = oracle.dequant_per_tensor(oracle.igemm(dense, B, threads=0), np.float32(0.011), np.float32(0.007))
+    assert np.array_equal(got[1:M + 1].view(np.uint32), want.view(np.uint32))
