@@ -784,16 +784,19 @@ int bm_quantize_rows_f16(const uint16_t* X_f16, int8_t* X_q, float* scale_m, int
     // Threads per row.  Many rows: four 16-byte pieces a thread, so that a 4096-wide row is one CTA of 128 threads with
     // 16 data registers each and an SM holds a dozen rows at different points of load, reduction and store.  Few
     // rows: one piece a thread while 1024 threads reach — the chip is empty and the length of a thread's own work is the
-    // latency.  (Launched in plain stream order on purpose: as a programmatic dependent of the GEMM before it the layer of 16
+    // latency.  Many rows of more than 16384 columns keep 512 threads and read the rest twice: 1024 threads with two pieces
+    // (50 registers) reach no further and leave an SM one row at a time (8192 x 16400 140.6 us against 79.3, 8192 x 32768
+    // 257.8 against 163.0, 149 x 16400 4.7 against 3.6; one warp per row 114, 284 and 15.4).  (Launched in plain stream order on purpose: as a programmatic dependent of the GEMM before it the layer of 16
     // tokens took 80.5 us instead of 78.1, the one of 8192 tokens 1163 instead of 1149.)
     const int vecs = K / 8;
     auto group_for = [&](int held) { return (ceil_div(vecs, held) + 31) / 32 * 32; };
     int held = 4, group = group_for(4);
-    if (M <= sms || group > 512) {
-        held = group_for(1) <= kQuantMaxThreads && M <= sms ? 1 : 2;
+    if (M <= sms) {
+        held = group_for(1) <= kQuantMaxThreads ? 1 : 2;
         group = group_for(held);
     }
-    if (group > kQuantMaxThreads) group = kQuantMaxThreads;        // the rest of such a row is read twice
+    const int most = held == 4 ? 512 : kQuantMaxThreads;
+    if (group > most) group = most;                                // the rest of such a row is read twice
     const dim3 block(group, group == 32 ? 4 : 1);
     const dim3 grid(ceil_div(M, static_cast<int>(block.y)));
     const __half* x = reinterpret_cast<const __half*>(X_f16);
