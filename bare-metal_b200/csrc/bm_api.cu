@@ -414,6 +414,11 @@ static int launch_sparse_pair_left(const CUtensorMap& mw, const CUtensorMap& me,
     return BM_OK;
 }
 
+// an output of 4-byte elements in the reference orientation that the pair kernel can store through TMA
+static bool left_out_tma(const void* out, long long ld) {
+    return aligned16(out) && (static_cast<size_t>(ld) * 4) % 16 == 0 && opt(OPT_TMA_STORE) != 0;
+}
+
 // Sets up and launches the pair kernel in the reference orientation.  `elem` = bytes per operand element
 // (1: int8, 2: fp16); K counts logical elements, the tensor maps are byte maps.
 static int sparse_pair_left(int epi, bool f16, const void* S_comp, const uint8_t* meta_tiled, const void* B, void* out,
@@ -449,7 +454,7 @@ static int sparse_pair_left(int epi, bool f16, const void* S_comp, const uint8_t
     // int8 8192^3 (14 waves) 303 -> 277, 4096^3 (4) 48.6 -> 46.4, but 2048 x 4096 x 4096 (2) 22.2 -> 23.5.
     const bool deep = f16 || pair_tiles > 2 * max_pairs;
     CUtensorMap map_o = map_w;                       // placeholder unless the output qualifies for TMA stores
-    if (p.epi.vec_ok && opt(OPT_TMA_STORE) != 0) {
+    if (left_out_tma(out, ld)) {
         if (int rc = make_tensor_map_out(&map_o, out, Cn, R, static_cast<size_t>(ld) * 4, 4, deep ? 64 : 128)) return rc;
         p.epi.tma_ok = 1;
     }
@@ -465,15 +470,23 @@ static int sparse_pair_left(int epi, bool f16, const void* S_comp, const uint8_t
 // fewer waves.  Lone CTAs -> pairs (waves) over 26 shapes of ragged and even sizes: 1.3 to 1.9 times faster wherever pairs
 // need fewer (5408 x 1616 x 1600 (4, 3) int8 31.0 -> 24.3 us, fp16 33.8 -> 25.9; 2528 x 1536 x 7648 (2, 1) 32.6 -> 19.9, 45.1 -> 27.4;
 // 5904 x 6736 x 768 (17, 9) 106 -> 54, 104 -> 54), and within 3 % of one another, either way, where both need the same
-// (1600 x 1200 x 6752 (1, 1) 26.6 -> 27.4, 28.0 -> 26.9; 4912 x 832 x 2560 (2, 2) 16.6 -> 16.9, 19.2 -> 19.1).  Tile width 224
-// forces pairs.
-static bool sparse_pair_left_wanted(int R, int Cn, const DeviceState* dev, int forced) {
+// (1600 x 1200 x 6752 (1, 1) 26.6 -> 27.4, 28.0 -> 26.9; 4912 x 832 x 2560 (2, 2) 16.6 -> 16.9, 19.2 -> 19.1).  `forced` = 224
+// (a selector: the tiles are 256 wide) forces pairs.
+// An output that TMA cannot store (base or pitch off 16 bytes) leaves element by element and that, not the MMAs, sets the
+// time, which pairs shorten only over many waves or along a long K.  Such outputs, lone CTAs -> pairs, int8 and fp16:
+// 8192 x 8192 x 64 (28, 14) 511 -> 453, 512 -> 454; 8192 x 4096 x 1024 (14, 7) 239 -> 227, 259 -> 242; 2048 x 4096 x 4096 (4, 2)
+// 64.6 -> 60.5, 80.1 -> 71.8; 560 x 7792 x 6880 (3, 2) 78.4 -> 71.2, 97.4 -> 87.6; but 4096 x 4096 x 256 (7, 4) 97.2 -> 101.2,
+// 98.0 -> 103.0; 3200 x 1808 x 224 (3, 2) 39.2 -> 48.4, 39.3 -> 48.3; 3760 x 608 x 192 (2, 1) 20.2 -> 26.5, 20.3 -> 27.0;
+// 4736 x 1184 x 4672 (3, 2) int8 55.0 -> 57.9.  `k_bytes` is K in bytes of the dense operand.
+static bool sparse_pair_left_wanted(int R, int Cn, long long k_bytes, bool tma_out, const DeviceState* dev, int forced) {
     if (forced == 224) return dev->sm_count >= 2;
     if (forced != 0 || dev->sm_count < 2 || opt(OPT_SPARSE_PAIR) == 0) return false;
     auto waves = [&](int rows, int cols, int slots) {
         return (static_cast<long long>(ceil_div(R, rows)) * ceil_div(Cn, cols) + slots - 1) / slots;
     };
-    return waves(256, SpPairCfg<true>::BN, dev->sm_count / 2) < waves(128, 128, dev->sm_count);
+    const long long pair = waves(256, SpPairCfg<true>::BN, dev->sm_count / 2), lone = waves(128, 128, dev->sm_count);
+    if (pair >= lone) return false;
+    return tma_out || pair >= 7 || k_bytes >= 6144 || (lone >= 2 * pair && k_bytes >= 1024);
 }
 
 // option "sparse_pair" = 0 keeps large sparse-weight problems on the single-CTA kernel (testing hook)
@@ -540,7 +553,7 @@ static int sparse_gemm(int mode, int epi, const int8_t* S_comp, const uint8_t* m
         return fail_msg(BM_ERR_LAYOUT, "unsupported epilogue for the sparse pair kernel");
     }
     if (bn == 240) bn = 0;
-    if (mode == 0 && dense_mn && !packed && sparse_pair_left_wanted(R, Cn, dev, bn))
+    if (mode == 0 && dense_mn && !packed && sparse_pair_left_wanted(R, Cn, K, left_out_tma(out, ld), dev, bn))
         return sparse_pair_left(epi, false, S_comp, meta_tiled, Dn, out, R, Cn, K, ld, tensor_scale, dev,
                                 static_cast<cudaStream_t>(stream_v));
     if (bn == 224) bn = 0;
@@ -915,7 +928,7 @@ int bm_hgemm_sparse_f32(const uint16_t* A_comp, const uint16_t* B, float* C, con
     if (int rc = current_device_state(&dev)) return rc;
     const int tiles_r = ceil_div(M, kBM);
     int bn = forced_bn();
-    if (sparse_pair_left_wanted(M, N, dev, bn))
+    if (sparse_pair_left_wanted(M, N, 2ll * K, left_out_tma(C, ldc), dev, bn))
         return sparse_pair_left(EPI_I32, true, A_comp, tiled, B, C, M, N, K, ldc, 1.f, dev, static_cast<cudaStream_t>(stream_v));
     // 128-column tiles: 4 stages and two accumulators fit; 256-column tiles leave room for 2 stages and
     // one accumulator only and were measured slower (4096^3: 122 vs 99 us; 8192^3: 904 vs 801 us)

@@ -187,6 +187,30 @@ __device__ __forceinline__ void drain_accumulator(const EpilogueParams& p, uint3
     }
 }
 
+struct NoHook {
+    __device__ __forceinline__ void operator()() const {}
+};
+
+// The same in the normal orientation, without column-side parameters: `reverse` drains the last chunk first, `first_read` is
+// called once, when the first chunk has left the accumulator.
+template <int EPI, int NC, class Hook>
+__device__ __forceinline__ void drain_rows_direct(const EpilogueParams& p, uint32_t taddr, int row, int col0, int col_limit,
+                                                  bool reverse, const Hook& first_read) {
+    static_assert(EPI == EPI_I32 || EPI == EPI_F32_TENSOR, "results without column parameters");
+    constexpr int CHUNKS = NC / 32;
+    auto chunk_at = [&](int i) { return reverse ? CHUNKS - 1 - i : i; };
+    auto live_at = [&](int i) { return col0 + chunk_at(i) * 32 < col_limit; };                 // warp-uniform
+    uint32_t rr[2][32];
+    if (live_at(0)) tmem_ld_32x32(taddr + chunk_at(0) * 32, rr[0]);
+#pragma unroll
+    for (int i = 0; i < CHUNKS; ++i) {
+        if (live_at(i)) tmem_ld_wait();
+        if (i == 0) first_read();
+        if (i + 1 < CHUNKS && live_at(i + 1)) tmem_ld_32x32(taddr + chunk_at(i + 1) * 32, rr[(i + 1) & 1]);
+        if (live_at(i)) emit_row_chunk<EPI>(p, row, col0 + chunk_at(i) * 32, rr[i & 1], nullptr, nullptr, 0.f);
+    }
+}
+
 // ------------------------------------------------------------------------------------------------
 // TMA-store drain (normal orientation).  Direct stores from the accumulator layout make every
 // lane of a warp write a different output ROW (16 bytes each, a pitch apart); with power-of-two
@@ -251,9 +275,6 @@ struct TmemSource {
 // read by its stores — what keeps the epilogue going when the stores go to other GPUs over NVLink.
 // `first_read` is called once, when the first chunk has left the accumulator; `reverse` (boxes of one chunk only) drains
 // the last chunk first.
-struct NoHook {
-    __device__ __forceinline__ void operator()() const {}
-};
 template <int EPI, int NC, int NBUF, class Source, class Hook = NoHook>
 __device__ __forceinline__ void drain_tma_from(const EpilogueParams& p, const CUtensorMap* maps, int n_maps, const Source& src,
                                                int row0, int lane, int col0, const EpiStrip<NC>* strip, float lane_s,

@@ -301,7 +301,7 @@ igemm_sparse_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
                 __syncwarp();
                 if (lane == 0) mbar_arrive_cluster(mapa_shared(overlap_bar, 0));
             };
-            bool stored = false;
+            [[maybe_unused]] bool stored = false;
             if constexpr (LEFT) {
                 if (p.epi.tma_ok) {
                     if constexpr (PC::NARROW)
@@ -315,9 +315,10 @@ igemm_sparse_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
                     stored = true;
                 }
             }
-            if (!stored) {
-                drain_accumulator<EPI, kSpPairNC, !LEFT>(p.epi, taddr, channel, t0, t_limit, strip, lane_s);
-                if constexpr (LEFT) overlap_read();
+            if constexpr (LEFT) {
+                if (!stored) drain_rows_direct<EPI, kSpPairNC>(p.epi, taddr, channel, t0, t_limit, half == 1, overlap_read);
+            } else {
+                drain_accumulator<EPI, kSpPairNC, true>(p.epi, taddr, channel, t0, t_limit, strip, lane_s);
             }
             tc_fence_before_sync();
             __syncwarp();

@@ -40,3 +40,24 @@ def test_pieces_a_thread_of_the_quantiser(M, K, pieces):
     x = torch.zeros((M, K), dtype=torch.float16, device=dev())
     names = captured_kernels(lambda: ig.quantize_rows(x, M, K))
     assert len(names) == 1 and f"quantize_rows_f16_kernelILi{pieces}E" in names[0]
+
+
+# three waves of lone CTAs against two of pairs; the same with a pitch and with a base that TMA cannot store; a K long
+# enough for pairs all the same; fourteen waves of pairs; one wave either way
+@pytest.mark.parametrize("M,N,K,pad,shift,pairs", [(3200, 1808, 224, 0, 0, True), (3200, 1808, 224, 1, 0, False),
+                                                   (3200, 1808, 224, 0, 1, False), (560, 7792, 6880, 1, 0, True),
+                                                   (8192, 8192, 32, 1, 0, True), (1600, 1200, 256, 0, 0, False)])
+def test_sparse_operand_on_the_left_with_outputs_that_tma_cannot_store(M, N, K, pad, shift, pairs):
+    def zeros(*shape, dtype, value=0):
+        return torch.full(shape, value, dtype=dtype, device=dev())
+    out = zeros(shift + M * (N + pad), dtype=torch.int32)[shift:].view(M, N + pad)[:, :N]
+    comp, B, meta = zeros(M, K // 2, dtype=torch.int8), zeros(K, N, dtype=torch.int8), zeros(M, K // 8, dtype=torch.uint8, value=0x44)
+    tiled = ig.sp_pack_meta(meta, ig.BM_META_ROWS, M, K)
+    names = captured_kernels(lambda: ig.igemm_sparse_i32(comp, tiled, ig.BM_META_TILED, B, out, M, N, K, ig.BM_B_KN))
+    assert len(names) == 1 and ("igemm_sparse_pair_kernel" in names[0]) == pairs
+    if K < 4096:                                       # half the K: the same bytes of an fp16 operand
+        half, dense = zeros(M, K // 4, dtype=torch.float16), zeros(K // 2, N, dtype=torch.float16)
+        f16_meta = ig.sp_pack_meta(zeros((M // 16) * (K // 32) * 8, dtype=torch.int32, value=0x44444444), ig.BM_META_REF_F16, M, K // 2)
+        c = out.view(torch.float32)
+        names = captured_kernels(lambda: ig.hgemm_sparse_tiled(half, dense, c, f16_meta, M, N, K // 2, ig.BM_META_TILED))
+        assert len(names) == 1 and ("igemm_sparse_pair_kernel" in names[0]) == pairs

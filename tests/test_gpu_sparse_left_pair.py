@@ -85,3 +85,20 @@ def test_scaled_fp32_results_where_the_launcher_chooses(M, N, K):
     assert (got[0] == -1).all() and (got[-1] == -1).all(), "store outside the output"
     want = oracle.dequant_per_tensor(oracle.igemm(dense, B, threads=0), np.float32(0.011), np.float32(0.007))
     assert np.array_equal(got[1:M + 1].view(np.uint32), want.view(np.uint32))
+
+
+@pytest.mark.parametrize("pad,shift", [(1, 0), (0, 1), (2, 3)])
+def test_integers_are_exact_where_outputs_leave_element_by_element(pad, shift):
+    """A pitch or base off 16 bytes, several tiles per pair: the chunk that both accumulators share leaves first."""
+    M, N, K = 2064, 6384, 96
+    comp, nib, dense = sparse_left(M, K, 6)
+    B = oracle.gen_int8((K, N), 6, 2)
+    tiled = ig.sp_pack_meta(nib, ig.BM_META_ROWS, M, K)
+    flat = torch.full((shift + M * (N + pad) + 8,), 0x5A5A5A5A, dtype=torch.int32, device=dev())
+    C = flat[shift:shift + M * (N + pad)].view(M, N + pad)[:, :N]
+    with options(force_bn=224):
+        ig.igemm_sparse_i32(comp, tiled, ig.BM_META_TILED, T(B), C, M, N, K, ig.BM_B_KN)
+        assert_clean_status()
+    assert np.array_equal(C.cpu().numpy(), oracle.igemm(dense, B, threads=0))
+    C.fill_(0x5A5A5A5A)
+    assert bool((flat == 0x5A5A5A5A).all()), "store outside the output"
