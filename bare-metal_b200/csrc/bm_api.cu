@@ -215,9 +215,12 @@ static int dense_gemm(int epi, const int8_t* A, const int8_t* B, void* C, int M,
         }
         pair_ok = best_pair;
     }
-    // Few tokens on weights [N x K]: channels on the lanes.  Up to 16 tokens always (the wide tiles spend 3 to 30 us on
-    // zero-filled token rows; 16 tokens, wide -> lanes: 4096 x 4096 14.3 -> 5.9 us, 12288 x 4096 21.4 -> 10.2, 22016 x 4096 32.7 ->
-    // 16.2, 4096 x 11008 18.7 -> 9.9, 28672 x 8192 41.6 -> 36.5), above that where the model sees it ahead (12288 x 4096, 96
+    // Few tokens on weights [N x K]: channels on the lanes.  Up to 16 tokens from K = 1024 on, 512 where there are 4096 channels,
+    // any where there are 8192 and the rows are off the 128-byte lines (the wide tiles spend up to 30 us on zero-filled token
+    // rows; 16 tokens, wide -> lanes: 4096 x 4096 14.3 -> 5.9 us, 12288 x 4096 21.4 -> 10.2, 22016 x 4096 32.7 -> 16.2, 4096 x 11008
+    // 18.7 -> 9.9, 28672 x 8192 41.6 -> 36.5, 1024 x 1024 3.4 -> 3.4, 4096 x 512 3.1 -> 2.8, 22016 x 272 6.3 -> 5.1; below, the
+    // launch is most of the time and theirs is shorter: 1024 x 64 2.15 -> 2.72, 1024 x 512 2.67 -> 3.25, 2048 x 768 3.09 -> 3.26,
+    // 8192 x 256 2.9 -> 3.4).  Above 16 tokens where the model sees it ahead (12288 x 4096, 96
     // tokens 12.7 -> 11.0; 4096 x 11008, 64 tokens 18.8 -> 13.3; but 128 tokens 19.2 against 21.5, and 1024 x 1024, 64
     // tokens 3.6 against 4.6).  The wide tiles also stream the weights more slowly than their own model says: 22016 x 4096,
     // 32 tokens 20.9 us for one wave.
@@ -225,7 +228,8 @@ static int dense_gemm(int epi, const int8_t* A, const int8_t* B, void* C, int M,
         const DenseDecodePlan plan = plan_dense_decode(M, N, K, dev->sm_count);
         const float stream_us = 2.8f + 1.35f * N * K / 6.8e6f;
         const float wide_us = tile_us > stream_us ? tile_us : stream_us;
-        if (opt(OPT_DENSE_DECODE) == 1 || (!bn_forced && (M <= 16 || plan.us < wide_us)))
+        const bool lanes = M > 16 ? plan.us < wide_us : K >= 1024 || (K >= 512 && N >= 4096) || (K % kBK != 0 && N >= 8192);
+        if (opt(OPT_DENSE_DECODE) == 1 || (!bn_forced && lanes))
             return dense_decode(epi, A, B, p.epi, M, N, K, plan, dev, static_cast<cudaStream_t>(stream_v));
     }
     if (b_mn && bn < 128) bn = 128;

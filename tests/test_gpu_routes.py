@@ -61,3 +61,14 @@ def test_sparse_operand_on_the_left_with_outputs_that_tma_cannot_store(M, N, K, 
         c = out.view(torch.float32)
         names = captured_kernels(lambda: ig.hgemm_sparse_tiled(half, dense, c, f16_meta, M, N, K // 2, ig.BM_META_TILED))
         assert len(names) == 1 and ("igemm_sparse_pair_kernel" in names[0]) == pairs
+
+
+# 16 tokens and few channels or a short K: the wide tiles
+@pytest.mark.parametrize("M,N,K,lanes", [(16, 1024, 64, False), (1, 512, 256, False), (8, 2048, 768, False), (16, 1024, 272, False),
+                                         (16, 4096, 512, True), (1, 16384, 768, True), (16, 64, 1024, True), (16, 1024, 1040, True),
+                                         (1, 22016, 272, True), (16, 8192, 256, False)])
+def test_few_tokens(M, N, K, lanes):
+    x, w = torch.zeros((M, K), dtype=torch.int8, device=dev()), torch.zeros((N, K), dtype=torch.int8, device=dev())
+    c = torch.zeros((M, N), dtype=torch.int32, device=dev())
+    names = captured_kernels(lambda: ig.igemm_i32(x, w, c, M, N, K, ig.BM_B_NK))
+    assert len(names) == 1 and ("igemm_dense_decode_kernel" in names[0]) == lanes
