@@ -81,9 +81,11 @@ struct DenseDecodePlan {
 // The fewest tiles per SM that fit, and the fold that needs the least tensor time.  `us` is a fit to W8A8 fp16-output
 // runs with 1 to 256 tokens over weights from 512 x 4096 to 28672 x 8192 (within ~15 %): launch, ramp and drain 3.2 us; the
 // longest of the weights at 6.8 TB/s, one SM's share of both operands at 105 KB/us, and the MMAs (57 clocks each at
-// least, half a clock per column from 114 columns up); the drain of the tokens.
+// least, half a clock per column where that is more); the drain of the tokens.  Where K is not whole blocks the rows are off
+// the 128-byte lines and every row of a box is two of them: an SM takes in 105 KB/us while few pull and 70 while all do
+// (128 tokens on 22016 x 8208 58 us, 64 on 1024 x 2064 7.1 against 5.5 on 1024 x 2048).
 static DenseDecodePlan plan_dense_decode(int M, int N, int K, int sms) {
-    const int bn = (M + 15) / 16 * 16, k_chunks = ceil_div(K, kBK);
+    const int bn = (M + 15) / 16 * 16, full_chunks = K / kBK, ragged = K % kBK != 0;
     const int groups = ceil_div(N, 8);                                           // channels in groups of 8
     const int waves = ceil_div(groups, kBM / 8 * sms);
     const int rows = ceil_div(groups, waves * sms) * 8;
@@ -91,12 +93,15 @@ static DenseDecodePlan plan_dense_decode(int M, int N, int K, int sms) {
     float mma = 0.f;
     for (int fold = 1; fold <= 8; fold *= 2) {
         // the folded epilogue is written for a CTA's only tile (tiles of a second wave have 72 channels or more and do not fit)
-        if (fold > 1 && (waves > 1 || rows * fold > kBM || bn * fold > 256 || rows * fold * bn > kDdPartInts || fold > k_chunks)) break;
-        const float us = static_cast<float>(waves) * ceil_div(k_chunks, fold) * 4.f *
-                         (bn * fold < 114 ? 57.f : bn * fold / 2.f) / 1.8e3f;
+        if (fold > 1 && (waves > 1 || rows * fold > kBM || bn * fold > 256 || rows * fold * bn > kDdPartInts || fold > full_chunks)) break;
+        const float us = static_cast<float>(waves) * 4.f * (ceil_div(full_chunks, fold) * (bn * fold < 114 ? 57.f : bn * fold / 2.f) +
+                                                            ragged * (bn < 114 ? 57.f : bn / 2.f)) / 1.8e3f;
         if (fold == 1 || us < mma) { mma = us; plan.fold = fold; }
     }
-    const float hbm = static_cast<float>(N) * K / 6.8e6f, fill = static_cast<float>(waves) * (rows + bn) * K / 105e3f;
+    const float hbm = static_cast<float>(N) * K / 6.8e6f;
+    float fill = static_cast<float>(waves) * (rows + bn) * K / 105e3f;
+    const int tiles = ceil_div(N, rows);
+    if (ragged) fill *= 1.f + 0.5f * (tiles < sms ? tiles : sms) / sms;
     float body = hbm > fill ? hbm : fill;
     if (mma > body) body = mma;
     plan.us = 3.2f + body + 0.008f * M;
@@ -124,26 +129,27 @@ static int dense_decode(int epi, const int8_t* X, const int8_t* W, const Epilogu
     p.acc_stride = (p.tokens_padded * p.fold + 31) / 32 * 32;
     p.tmem_cols = 64;
     while (p.tmem_cols < 2 * p.acc_stride) p.tmem_cols *= 2;
-    const int k_chunks = ceil_div(K, kBK), group_bytes = (p.tile_rows + p.tokens_padded) * kBK * p.fold;
+    const int group_bytes = (p.tile_rows + p.tokens_padded) * kBK * p.fold;
     p.full_chunks = K / kBK;
-    p.whole_chunks = K % kBK == 0;
+    const bool ragged = K % kBK != 0;
     int per_stage = ceil_div(16 * 1024, group_bytes);            // stages of at least 16 KiB
-    if (per_stage > ceil_div(k_chunks, p.fold)) per_stage = ceil_div(k_chunks, p.fold);
+    const int groups = p.full_chunks > 0 ? ceil_div(p.full_chunks, p.fold) : 1;
+    if (per_stage > groups) per_stage = groups;
     p.chunks = per_stage * p.fold;
     p.stages = kDdRingBytes / (per_stage * group_bytes);
     if (p.stages > kDdMaxStages) p.stages = kDdMaxStages;
-    p.k_stages = ceil_div(k_chunks, p.chunks);
+    p.full_stages = ceil_div(p.full_chunks, p.chunks);
+    p.k_stages = p.full_stages + ragged;
     p.status = dev->status;
     CUtensorMap w2, x2, w3, x3;                                  // a pair that no stage takes is a copy of the other
-    const bool any3 = p.whole_chunks || p.full_chunks >= p.chunks;
-    if (any3) {
+    if (p.full_chunks > 0) {
         if (int rc = make_tensor_map_kblocks(&w3, W, p.full_chunks, N, K, p.tile_rows, p.chunks)) return rc;
         if (int rc = make_tensor_map_kblocks(&x3, X, p.full_chunks, M, K, p.tokens_padded, p.chunks)) return rc;
     }
-    if (!p.whole_chunks) {                                       // a ragged last K block
+    if (ragged) {
         if (int rc = make_tensor_map_u8(&w2, W, K, N, K, kBK, p.tile_rows, true)) return rc;
         if (int rc = make_tensor_map_u8(&x2, X, K, M, K, kBK, p.tokens_padded, true)) return rc;
-        if (!any3) { w3 = w2; x3 = x2; }
+        if (p.full_chunks == 0) { w3 = w2; x3 = x2; }
     } else {
         w2 = w3;
         x2 = x3;
@@ -223,10 +229,12 @@ static int dense_gemm(int epi, const int8_t* A, const int8_t* B, void* C, int M,
     // 8192 x 256 2.9 -> 3.4).  Above 16 tokens where the model sees it ahead (12288 x 4096, 96
     // tokens 12.7 -> 11.0; 4096 x 11008, 64 tokens 18.8 -> 13.3; but 128 tokens 19.2 against 21.5, and 1024 x 1024, 64
     // tokens 3.6 against 4.6).  The wide tiles also stream the weights more slowly than their own model says: 22016 x 4096,
-    // 32 tokens 20.9 us for one wave.
+    // 32 tokens 20.9 us for one wave; with rows off the lines 22016 x 8208 takes 45.6, and 96 tokens on 8192 x 8208 27.
     if (!b_mn && n_peers == 0 && M <= kDdMaxTokens && epi != EPI_F32_ROWCOL && opt(OPT_DENSE_DECODE) != 0) {
         const DenseDecodePlan plan = plan_dense_decode(M, N, K, dev->sm_count);
-        const float stream_us = 2.8f + 1.35f * N * K / 6.8e6f;
+        const float ragged_k = K % kBK != 0 ? static_cast<float>(K) : 0.f;
+        const float stream_us = 2.8f + (ragged_k == 0.f ? 1.35f : 1.62f) * N * K / 6.8e6f;
+        tile_us *= 1.f + 0.2f * ragged_k / 8192.f;
         const float wide_us = tile_us > stream_us ? tile_us : stream_us;
         const bool lanes = M > 16 ? plan.us < wide_us : K >= 1024 || (K >= 512 && N >= 4096) || (K % kBK != 0 && N >= 8192);
         if (opt(OPT_DENSE_DECODE) == 1 || (!bn_forced && lanes))

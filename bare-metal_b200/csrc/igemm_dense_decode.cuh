@@ -8,8 +8,8 @@
 // SMs; N = 12288: 88 on 140).  The MMA always spans 128 lanes; what it reads beyond the tile's h rows (other
 // ring bytes) lands in lanes nobody stores.  Tokens are the accumulator columns, rounded up to 16.
 //
-// An MMA takes at least 57 clocks however few tokens it has (measured with the operands resident; from 128
-// columns on it is half a clock per column), so K = 4096 in steps of 32 is 3.9 us of MMAs — more than
+// An MMA takes at least 57 clocks however few tokens it has (measured with the operands resident; half a clock per
+// column where that is more), so K = 4096 in steps of 32 is 3.9 us of MMAs — more than
 // the 2.6 us that 4096 x 4096 weights take from HBM.  Tiles of at most 64 channels therefore FOLD K: the
 // stage's chunks lie in shared memory one after the other, [chunk][h rows][128 B], which is also a
 // matrix of chunk * h rows; `fold` chunks of W stacked on the 128 lanes against `fold` chunks of X stacked on
@@ -20,9 +20,11 @@
 //
 // A ring stage covers `chunks` K blocks of 128 bytes, a multiple of `fold`.  W and X are described to the TMA as
 // [K / 128][rows][128 B], so one copy fetches all chunks of an operand's stage: a 32-row box of one chunk is only
-// 4 KiB.  The last, ragged chunk of a K that is not a multiple of 128 comes through a plain 2-D map instead, which
-// zero-fills beyond K (chunks that do not exist arrive as zeros either way).  All stage geometry is a launch
-// parameter: one instantiation per epilogue.
+// 4 KiB (chunks that do not exist arrive as zeros).  The ragged chunk of a K that is not a multiple of 128 is a stage of its
+// own, the last of every tile: one copy per operand through a plain 2-D map, which zero-fills beyond K, and MMAs without
+// folding, whose sums join those of the first K range.  (As part of the last stage it took a copy per chunk of that stage
+// and operand and a folded MMA for the one chunk: 1024 x 1040 with 16 / 32 tokens 5.1 / 5.3 us against 4.3 / 4.7.)  All
+// stage geometry is a launch parameter: one instantiation per epilogue.
 //
 // What bounds it: the weights' stream from HBM (28672 x 8192, 1 token: 35.5 us = 6.6 TB/s) plus ~3.2 us of launch, ramp and
 // drain; with many tokens what one SM can take in of both operands.  16 tokens, before (wide tiles) -> without folding ->
@@ -56,8 +58,8 @@ struct DenseDecodeParams {
     int fold;                          // K blocks side by side in one MMA (1: none); above 1 only with tiles <= grid
     int acc_stride, tmem_cols;         // columns between the two accumulators; columns allocated
     int chunks, stages;                // K blocks of 128 bytes per ring stage; ring stages
-    int full_chunks, whole_chunks;     // K blocks entirely inside K; 1: there are no others (K % 128 == 0)
-    int k_stages;                      // stages that cover K
+    int full_chunks;                   // K blocks entirely inside K
+    int full_stages, k_stages;         // stages that cover these; one more where K ends inside a block
     int* status;
 };
 
@@ -90,8 +92,8 @@ igemm_dense_decode_kernel(const __grid_constant__ CUtensorMap map_w3, const __gr
     const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0);      // known to be the same in all lanes
     const int lane = threadIdx.x & 31;
     const uint32_t nstages = static_cast<uint32_t>(p.stages);
-    const int rot = static_cast<int>((blockIdx.x * 7u) % static_cast<unsigned>(p.k_stages));
-    auto k_stage_of = [&](int i) { const int k = i + rot; return k < p.k_stages ? k : k - p.k_stages; };
+    const int rot = p.full_stages > 0 ? static_cast<int>((blockIdx.x * 7u) % static_cast<unsigned>(p.full_stages)) : 0;
+    auto k_stage_of = [&](int i) { const int k = i + rot; return k < p.full_stages ? k : k - p.full_stages; };
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < p.stages; ++s) {
@@ -124,24 +126,24 @@ igemm_dense_decode_kernel(const __grid_constant__ CUtensorMap map_w3, const __gr
         const CUtensorMap* map3 = is_w ? &map_w3 : &map_x3;
         const CUtensorMap* map2 = is_w ? &map_w2 : &map_x2;
         prefetch_tensormap(map3);
+        if (p.k_stages > p.full_stages) prefetch_tensormap(map2);
         const uint32_t base = is_w ? w_smem0 : x_smem0, stage_bytes = is_w ? w_stage : x_stage;
-        const uint32_t chunk_bytes = is_w ? w_chunk : x_chunk;
         uint32_t stage = 0, phase = 0;
         bool ok = true;
         for (int tile = blockIdx.x; ok && tile < p.tiles; tile += gridDim.x) {
             const int row0 = is_w ? tile * p.tile_rows : 0;
             for (int i = 0; i < p.k_stages; ++i) {
-                const int ks = k_stage_of(i), c0 = ks * p.chunks;
                 if (!warp_bounded_wait(empty_bar(stage), phase ^ 1u, abort_flag, p.status,
                                   DEV_TIMEOUT_PRODUCER_EMPTY)) { ok = false; break; }
                 const uint32_t bar = full_bar(stage);
                 const uint32_t dst = base + stage * stage_bytes;
                 if (elect_one()) {
-                    if (is_w) mbar_expect_tx(bar, w_stage + x_stage);   // both operands
-                    if (p.whole_chunks || c0 + p.chunks <= p.full_chunks) {
-                        tma_load_3d(dst, map3, bar, 0, row0, c0);
+                    if (i < p.full_stages) {
+                        if (is_w) mbar_expect_tx(bar, w_stage + x_stage);   // both operands
+                        tma_load_3d(dst, map3, bar, 0, row0, k_stage_of(i) * p.chunks);
                     } else {
-                        for (int c = 0; c < p.chunks; ++c) tma_load_2d(dst + c * chunk_bytes, map2, bar, (c0 + c) * 128, row0);
+                        if (is_w) mbar_expect_tx(bar, w_chunk + x_chunk);
+                        tma_load_2d(dst, map2, bar, p.full_chunks * 128, row0);
                     }
                 }
                 __syncwarp();
@@ -151,6 +153,7 @@ igemm_dense_decode_kernel(const __grid_constant__ CUtensorMap map_w3, const __gr
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
         const uint32_t idesc = make_idesc_i8(kBM, p.tokens_padded * p.fold, false, false);
+        const uint32_t idesc_ragged = make_idesc_i8(kBM, p.tokens_padded, false, false);
         const uint64_t w_desc0 = make_smem_desc(w_smem0, 0, 1024, SWIZZLE_128B_DESC);
         const uint64_t x_desc0 = make_smem_desc(x_smem0, 0, 1024, SWIZZLE_128B_DESC);
         uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
@@ -161,7 +164,7 @@ igemm_dense_decode_kernel(const __grid_constant__ CUtensorMap map_w3, const __gr
             tc_fence_after_sync();
             const uint32_t d_tmem = tmem_base + acc * p.acc_stride;
             uint32_t accumulate = 0u;
-            for (int i = 0; i < p.k_stages; ++i) {
+            for (int i = 0; i < p.full_stages; ++i) {
                 if (!warp_bounded_wait(full_bar(stage), phase, abort_flag, p.status, DEV_TIMEOUT_MMA_FULL)) {
                     ok = false;
                     break;
@@ -185,6 +188,23 @@ igemm_dense_decode_kernel(const __grid_constant__ CUtensorMap map_w3, const __gr
                 if (++stage == nstages) { stage = 0; phase ^= 1u; }
             }
             if (!ok) break;
+            if (p.k_stages > p.full_stages) {                        // the ragged chunk
+                if (!warp_bounded_wait(full_bar(stage), phase, abort_flag, p.status, DEV_TIMEOUT_MMA_FULL)) {
+                    ok = false;
+                    break;
+                }
+                tc_fence_after_sync();
+                if (elect_one()) {
+                    const uint64_t a_desc = w_desc0 + ((stage * w_stage) >> 4), b_desc = x_desc0 + ((stage * x_stage) >> 4);
+#pragma unroll
+                    for (int s = 0; s < kBK / kUmmaK; ++s)
+                        mma_i8(d_tmem, a_desc + s * (kUmmaK >> 4), b_desc + s * (kUmmaK >> 4), idesc_ragged,
+                               s != 0 ? 1u : accumulate);
+                    tc_commit(empty_bar(stage));
+                }
+                __syncwarp();
+                if (++stage == nstages) { stage = 0; phase ^= 1u; }
+            }
             if (elect_one()) tc_commit(acc_full_bar(acc));
             __syncwarp();
             acc ^= 1u;

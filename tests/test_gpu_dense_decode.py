@@ -13,7 +13,9 @@ pytestmark = pytest.mark.gpu
 # that do not exist; token counts at the 16- and 32-column borders up to the largest
 SHAPES = [(1, 8, 16), (1, 9, 128), (16, 1184, 144), (17, 2368, 1024), (31, 1192, 2064), (33, 4096, 528), (48, 300, 4112),
           (64, 4104, 1024), (65, 640, 256), (100, 12296, 272), (127, 1000, 1152), (128, 4096, 640), (129, 96, 2048),
-          (255, 2376, 400), (256, 19000, 160)]
+          (255, 2376, 400), (256, 19000, 160),
+          # the ragged K block after folded ones: one, a part of a group, whole groups
+          (5, 64, 144), (16, 600, 432), (16, 1024, 1040), (64, 2048, 2064), (3, 1184, 1136)]
 
 
 @pytest.mark.parametrize("M,N,K", SHAPES)

@@ -63,10 +63,13 @@ def test_sparse_operand_on_the_left_with_outputs_that_tma_cannot_store(M, N, K, 
         assert len(names) == 1 and ("igemm_sparse_pair_kernel" in names[0]) == pairs
 
 
-# 16 tokens and few channels or a short K: the wide tiles
+# 16 tokens and few channels or a short K: the wide tiles; from 17 tokens on weights whose rows are off the 128-byte lines: wide
+# tiles where all SMs pull both operands
 @pytest.mark.parametrize("M,N,K,lanes", [(16, 1024, 64, False), (1, 512, 256, False), (8, 2048, 768, False), (16, 1024, 272, False),
                                          (16, 4096, 512, True), (1, 16384, 768, True), (16, 64, 1024, True), (16, 1024, 1040, True),
-                                         (1, 22016, 272, True), (16, 8192, 256, False)])
+                                         (1, 22016, 272, True), (16, 8192, 256, False),
+                                         (32, 1024, 1040, False), (64, 2048, 2064, False), (96, 1024, 4112, False),
+                                         (128, 22016, 4112, False), (17, 64, 4112, True), (32, 4096, 4112, True)])
 def test_few_tokens(M, N, K, lanes):
     x, w = torch.zeros((M, K), dtype=torch.int8, device=dev()), torch.zeros((N, K), dtype=torch.int8, device=dev())
     c = torch.zeros((M, N), dtype=torch.int32, device=dev())
