@@ -2,6 +2,7 @@
 // Argument validation, tensor-map encoding, tile-shape choice and the kernel launch; no
 // arithmetic happens on the host.
 #include <cstdlib>
+#include <type_traits>
 
 #include "host_common.cuh"
 #include "igemm_dense.cuh"
@@ -858,11 +859,19 @@ int bm_online_quant_gemm_f32(const uint16_t* A_f16, const uint16_t* B_f16, float
     float* row_scale = reinterpret_cast<float*>(ws);            ws += up(sizeof(float) * M);
     float* col_scale = reinterpret_cast<float*>(ws);            ws += up(sizeof(float) * N);
     const int blocks_a = ceil_div(M, kOqRowBlock), blocks_b = ceil_div(N, col_block);
-    const int a_per = ceil_div(K, 256), b_per = ceil_div(K, kOqChunkElems / col_block);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    oq_quantize_kernel<<<blocks_a * a_per + blocks_b * b_per, kOqThreads, 0, st>>>(
-        reinterpret_cast<const __half*>(A_f16), reinterpret_cast<const __half*>(B_f16), Aq, Bq, row_scale, col_scale, M,
-        N, K, col_block, blocks_a * a_per, a_per, b_per);
+    auto quantise = [&](auto threads) {                // false: more CTAs than the SMs hold at once
+        constexpr int T = decltype(threads)::value;
+        const int a_per = ceil_div(K, OqCfg<T>::A_COLS), b_per = ceil_div(K, OqCfg<T>::CHUNK / col_block);
+        const long long ctas = static_cast<long long>(blocks_a) * a_per + static_cast<long long>(blocks_b) * b_per;
+        if (T == 512 && ctas > static_cast<long long>(dev->sm_count) * (kOqResidentThreads / T)) return false;
+        oq_quantize_kernel<T><<<static_cast<unsigned>(ctas), T, 0, st>>>(
+            reinterpret_cast<const __half*>(A_f16), reinterpret_cast<const __half*>(B_f16), Aq, Bq, row_scale, col_scale, M,
+            N, K, col_block, blocks_a * a_per, a_per, b_per);
+        return true;
+    };
+    // one wave of the larger chunks, else the smaller ones (see oq_quantize_kernel)
+    if (!quantise(std::integral_constant<int, 512>{})) quantise(std::integral_constant<int, 256>{});
     BM_CUDA_TRY(cudaGetLastError());
     return dense_gemm(EPI_F32_ROWCOL, Aq, Bq, C, M, N, K, N, BM_B_KN, 1.f, row_scale, col_scale, nullptr, stream);
 }

@@ -22,19 +22,32 @@ namespace bm {
 constexpr int kOqRowBlock = 128;
 constexpr int kOqKTile = 32;
 
-// One launch does both steps.  A CTA owns a chunk of 32768 elements inside ONE scale block — 128 rows x
-// 256 columns of A, or 256 (128) rows x 128 (256) columns of B.  It asks for its whole chunk first, 64 elements a
-// thread in registers, then takes the block's maximum over the first K tile itself (4096 / 8192 elements, an
+// One launch does both steps.  A CTA of 512 (256) threads owns a chunk of 32768 (16384) elements inside ONE scale block —
+// 128 rows x 256 (128) columns of A, or 256 or 128 (128 or 64) rows x 128 or 256 columns of B.  It asks for its whole chunk
+// first, 64 elements a thread in registers, then takes the block's maximum over the first K tile itself (4096 / 8192 elements, an
 // L2 hit for all but the first CTA of a block) while those loads are under way, and converts: two
 // 16-byte loads and one 16-byte store per 16 elements.  The CTAs of chunk 0 also publish the dequantisation scale
 // max / 127 per row / column for the GEMM epilogue.
 // K % 16 == 0 and N % 16 == 0, so a 16-element unit never straddles an edge.
 // Bound by HBM: 3 bytes per element (the GEMM behind it takes the rest of the time at the larger sizes).  With both steps,
 // before (256 threads, loads after the maximum, conversions of ~14 instructions an element) -> now: 256^3 10.2 ->
-// 7.7 us, 512 x 512 x 4096 15.7 -> 13.3, 8192 x 512 x 512 14.8 -> 12.5, 8192 x 4096 x 1024 58.7 -> 52.6, 4096^3 74.0 -> 72.7.
-constexpr int kOqChunkElems = 32768;
-constexpr int kOqThreads = 512;
-constexpr int kOqUnits = kOqChunkElems / 16 / kOqThreads;      // 16-element units a thread holds
+// 7.7 us, 512 x 512 x 4096 15.7 -> 13.3, 8192 x 512 x 512 14.8 -> 12.5, 4096^3 (the GEMM under the power cap) 73.4 -> 69.3.
+//
+// With 62 registers a thread an SM holds 1024 threads.  Chunks of 32768 are for what the SMs take in at once: beyond that,
+// CTAs of 512 threads came in waves of which the last was partly empty, and the call was slower than with the 256 threads
+// that loaded after the maximum.  Those, 512 threads, 256 threads now: 8192 x 512 x 8192 69.7, 72.7, 66.5 us; 3000 x 1024 x
+// 8192 48.5, 50.0, 46.4; 8192 x 512 x 4096 39.1, 41.2, 37.1; 8192 x 1024 x 8192 92.6, 94.6, 89.1; 4096^3 73.4, 71.9, 69.3.
+// Within one wave the larger chunks read the maximum's window less often: 4096 x 16 x 2048 15.7 against 17.3, 8192 x 16 x 1024
+// 17.4 against 18.5.
+constexpr int kOqUnits = 4;                                    // 16-element units a thread holds
+constexpr int kOqResidentThreads = 1024;                       // of an SM, with the registers that takes
+template <int THREADS>
+struct OqCfg {
+    static constexpr int CHUNK = THREADS * kOqUnits * 16;
+    static constexpr int A_COLS = CHUNK / kOqRowBlock;
+    static constexpr int A_UNITS_LOG = A_COLS == 256 ? 4 : 3;  // units of a chunk's row of A
+    static_assert(A_COLS == 256 || A_COLS == 128, "chunk of A");
+};
 
 struct OqUnit {
     uint4 lo, hi;
@@ -91,11 +104,13 @@ __device__ __forceinline__ uint4 oq_unit_convert(const OqUnit& u, float inv) {
     return make_uint4(out[0], out[1], out[2], out[3]);
 }
 
-__global__ void __launch_bounds__(kOqThreads, 2)
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS, kOqResidentThreads / THREADS)
 oq_quantize_kernel(const __half* __restrict__ A, const __half* __restrict__ B, int8_t* __restrict__ Aq,
                    int8_t* __restrict__ Bq, float* __restrict__ row_scale, float* __restrict__ col_scale, int M, int N,
                    int K, int col_block, int chunks_a, int a_chunks_per_block, int b_chunks_per_block) {
-    __shared__ float warp_max[kOqThreads / 32];
+    using Cfg = OqCfg<THREADS>;
+    __shared__ float warp_max[THREADS / 32];
     pdl_launch_dependents();      // the GEMM behind this kernel may start its own set-up
     const int kt = K < kOqKTile ? K : kOqKTile;
     const int tid = threadIdx.x;
@@ -108,15 +123,15 @@ oq_quantize_kernel(const __half* __restrict__ A, const __half* __restrict__ B, i
     const __half* X = is_a ? A : B;
     int8_t* Xq = is_a ? Aq : Bq;
     const int rows = is_a ? M : K, cols = is_a ? K : N;
-    const int units_log = is_a || col_block == 256 ? 4 : 3;
-    const int ch_rows = (kOqChunkElems / 16) >> units_log;
-    const int r0 = is_a ? blk * kOqRowBlock : chunk * ch_rows, c0 = is_a ? chunk * 256 : blk * col_block;
+    const int units_log = is_a ? Cfg::A_UNITS_LOG : col_block == 256 ? 4 : 3;
+    const int ch_rows = (Cfg::CHUNK / 16) >> units_log;
+    const int r0 = is_a ? blk * kOqRowBlock : chunk * ch_rows, c0 = is_a ? chunk * Cfg::A_COLS : blk * col_block;
     const int w_r0 = is_a ? r0 : 0, w_c0 = is_a ? 0 : c0;
     const int w_rows = is_a ? kOqRowBlock : kt, w_cols = is_a ? kt : col_block;
 
     // a thread's units lie below one another, `step` rows apart
     const int first_r = r0 + (tid >> units_log), my_c = c0 + (tid & ((1 << units_log) - 1)) * 16;
-    const int step = kOqThreads >> units_log;
+    const int step = THREADS >> units_log;
     const int mine = my_c < cols ? rows - first_r : 0;     // unit i exists if i * step < mine
     const size_t at = static_cast<size_t>(first_r) * cols + my_c, pitch = static_cast<size_t>(step) * cols;
     OqUnit held[kOqUnits];
@@ -126,7 +141,7 @@ oq_quantize_kernel(const __half* __restrict__ A, const __half* __restrict__ B, i
 
     const int w_log = is_a ? 1 : units_log;               // window units per row: 2 (of which K < 32 has one) or those of the chunk
     float m = 0.f;
-    for (int u = tid; u < w_rows << w_log; u += kOqThreads) {
+    for (int u = tid; u < w_rows << w_log; u += THREADS) {
         const int r = w_r0 + (u >> w_log), c = w_c0 + (u & ((1 << w_log) - 1)) * 16;
         if (r < rows && c < cols && c < w_c0 + w_cols) m = fmaxf(m, oq_unit_max(oq_load(X + static_cast<size_t>(r) * cols + c)));
     }
@@ -136,13 +151,13 @@ oq_quantize_kernel(const __half* __restrict__ A, const __half* __restrict__ B, i
     __syncthreads();
     float bmax = warp_max[0];
 #pragma unroll
-    for (int w = 1; w < kOqThreads / 32; ++w) bmax = fmaxf(bmax, warp_max[w]);
+    for (int w = 1; w < THREADS / 32; ++w) bmax = fmaxf(bmax, warp_max[w]);
     const float inv = bmax > 0.f ? __fdiv_rn(127.0f, bmax) : 1.0f;
     if (chunk == 0) {
         const float scale = __fdiv_rn(bmax, 127.0f);
         float* dst = is_a ? row_scale : col_scale;
         const int first = is_a ? r0 : c0, count = is_a ? kOqRowBlock : col_block, limit = is_a ? M : N;
-        for (int i = tid; i < count; i += kOqThreads)
+        for (int i = tid; i < count; i += THREADS)
             if (first + i < limit) dst[first + i] = scale;
     }
 #pragma unroll

@@ -31,7 +31,9 @@ def quantise(x, axis_block, first_k, k_axis):
 
 # K of half a tile, below and above a chunk of A (256); rows and columns around the blocks and the rows of a chunk
 @pytest.mark.parametrize("M,N,K,col_block", [(1, 16, 16, 128), (127, 144, 48, 128), (129, 272, 256, 256), (130, 400, 272, 128),
-                                             (257, 112, 528, 256)])
+                                             (257, 112, 528, 256),
+                                             # more CTAs than fit at once: chunks of half the size
+                                             (130, 4112, 2320, 128), (2500, 272, 4112, 256)])
 def test_block_quantised_product_with_outliers(M, N, K, col_block):
     rng = np.random.default_rng(M * N + K)
     A = rng.uniform(-1, 1, (M, K)).astype(np.float16)

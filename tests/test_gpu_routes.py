@@ -75,3 +75,13 @@ def test_few_tokens(M, N, K, lanes):
     c = torch.zeros((M, N), dtype=torch.int32, device=dev())
     names = captured_kernels(lambda: ig.igemm_i32(x, w, c, M, N, K, ig.BM_B_NK))
     assert len(names) == 1 and ("igemm_dense_decode_kernel" in names[0]) == lanes
+
+
+# 296 CTAs of 512 threads are in flight at once on 148 SMs; more run as CTAs of 256
+@pytest.mark.parametrize("M,N,K,threads", [(256, 256, 256, 512), (4096, 16, 2048, 512), (4096, 4096, 1024, 512),
+                                           (4096, 4096, 2048, 256), (8192, 512, 4096, 256)])
+def test_threads_of_the_quantiser_of_fp16_operands(M, N, K, threads):
+    a, b = torch.zeros((M, K), dtype=torch.float16, device=dev()), torch.zeros((K, N), dtype=torch.float16, device=dev())
+    c = torch.zeros((M, N), dtype=torch.float32, device=dev())
+    names = captured_kernels(lambda: ig.igemm_online_quant(a, b, c, M, N, K))
+    assert len(names) == 2 and any(f"oq_quantize_kernelILi{threads}E" in n for n in names)
