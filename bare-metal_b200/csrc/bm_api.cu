@@ -202,8 +202,9 @@ static int dense_gemm(int epi, const int8_t* A, const int8_t* B, void* C, int M,
         // The per-wave figures (us at K = 4096, W8A8 fp16 out, one B200) were measured on problems from
         // 64 x 512 to 4352 x 8192: narrow tiles move more operand bytes per MAC but finish a wave sooner,
         // so they win while the wide tiles would leave SMs idle, and lose once they need a second wave.
-        // (The order of the candidates was measured with these; few_wave / few_start say what one of them takes by itself
-        // with few tokens, for the comparison with the channels-on-lanes kernel below.)
+        // (wave_us / start_us date from the slower issue of a divergent lane and order the candidates; few_wave / few_start
+        // were measured since and say what one of them takes by itself with few tokens, for the comparison with the
+        // channels-on-lanes kernel below.)
         struct Cand { int bn; bool pair; float wave_us, start_us, few_wave, few_start; };
         const Cand cands[4] = {{256, true, 12.0f, 3.6f, 12.0f, 3.4f}, {256, false, 12.3f, 3.0f, 13.5f, 2.8f},
                                {128, false, 9.8f, 2.8f, 7.8f, 2.6f}, {64, false, 9.3f, 2.6f, 6.0f, 2.4f}};
@@ -306,9 +307,9 @@ static int dense_gemm(int epi, const int8_t* A, const int8_t* B, void* C, int M,
         if (opt(OPT_DENSE_GROUP_M) >= 0) p.group_m = opt(OPT_DENSE_GROUP_M);
         // Half-height tail: when at most half of the pairs would work in the last wave, its tiles are
         // computed as two 128 x 256 halves by different pairs (M = 128 pair MMAs, 64 rows per CTA; no
-        // reduction).  Worth only ~1 % (4096^3: 48.1 -> 47.8 us): a K = 32 MMA step chained on one
-        // accumulator takes ~128 clocks whether it is 256 x 256, 256 x 128 or 128 x 256, so a smaller unit
-        // saves operand waits, not MMA time.  Option "tail_narrow" = 0 switches it off.  (Cutting the tail
+        // reduction).  Half units -> whole tiles, [N x K] and [K x N]: 2500 x 2256 x 2064 16.8 -> 19.0 us, 20.0 -> 22.4;
+        // 2304 x 2304 x 2048 12.7 -> 14.7, 14.7 -> 16.9; 5008 x 3008 x 2048 26.1 -> 29.0, 32.1 -> 35.3; no difference where
+        // the power cap holds the clock (4096^3, 8192 x 12288 x 4096).  Option "tail_narrow" = 0 switches it off.  (Cutting the tail
         // tiles along K instead — partial sums parked in global memory, last arrival finishes — was
         // measured 15 % SLOWER at 4096^3, 69.5 vs 60.3 us, and is not built.)
         {

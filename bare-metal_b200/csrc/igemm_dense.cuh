@@ -1,9 +1,9 @@
 // igemm_dense.cuh — dense INT8 GEMM for sm_100a: s8 x s8 -> s32 on the tcgen05 tensor cores.
 //
 // One persistent CTA per SM walks output tiles of 128 x BN.  Three warp roles:
-//   warp 0      TMA producer  — one lane streams 128-byte-swizzled operand tiles into a
+//   warp 0      TMA producer  — an elected lane streams 128-byte-swizzled operand tiles into a
 //                               ring of shared-memory stages (mbarrier full/empty pairs)
-//   warp 1      MMA issuer    — one lane issues tcgen05.mma.kind::i8 (M=128, N=BN, K=32),
+//   warp 1      MMA issuer    — an elected lane issues tcgen05.mma.kind::i8 (M=128, N=BN, K=32),
 //                               four per stage; accumulators live in tensor memory, two of
 //                               them, so tile t+1 accumulates while tile t is drained
 //   warps 2..9  epilogue      — two warps per tensor-memory lane quarter, each draining half of

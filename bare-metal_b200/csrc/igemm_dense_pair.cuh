@@ -3,7 +3,7 @@
 // Two CTAs of a 2-CTA cluster (two neighbouring SMs) compute one 256 x 256 output tile.  CTA r
 // of the pair owns accumulator rows [128 r, 128 r + 128) in ITS tensor memory and stages, per
 // K block, only ITS halves of the operands: 128 rows of A and 128 of the 256 columns of B.
-// The MMA, issued by one lane of the leader CTA (rank 0), reads A from each CTA's own shared
+// The MMA, issued by an elected lane of the leader CTA's issuer warp (rank 0), reads A from each CTA's own shared
 // memory and the two B halves from both.  Per SM and K byte that is 256 operand bytes for
 // 32768 MACs (4 tensor clocks) — 64 B/clk, against 96 B/clk for a lone 128 x 256 CTA, whose
 // measured fill rate (~65 B/clk/SM) is what caps it.  No copy is multicast: each CTA issues

@@ -10,8 +10,8 @@
 // The row is read once (16-byte loads, kept in registers while the maximum is reduced) and written once:
 // 3 bytes of HBM traffic per element, which bound it from a few hundred rows up; below that it is one memory round
 // trip plus a thread's own work.  Measured back to back on inputs beyond L2, against one warp per row with the row in its
-// registers (16 warps an SM, rows beyond 4096 read twice): 8192 x 4096 21.1 -> 16.5 us (6.1 TB/s), 8192 x 11008
-// 70.1 -> 44.4, 777 x 11008 15.3 -> 6.7, 16 x 4096 3.8 -> 1.5, 16 x 11008 9.0 -> 2.0.
+// registers (16 warps an SM, rows beyond 4096 read twice): 8192 x 4096 21.0 -> 17.0 us (5.9 TB/s; 18.7 in bench.py), 8192 x
+// 11008 70.2 -> 45, 777 x 11008 15.2 -> 7.3, 16 x 4096 3.8 -> 1.9, 16 x 11008 9.0 -> 2.4.
 #pragma once
 #include <cstdint>
 #include <cuda_fp16.h>

@@ -250,7 +250,8 @@ int bm_w8a8_sparse_f16_packed(const int8_t *X, const void *W_packed, uint16_t *D
 int bm_last_device_status(int *code);
 /* Launcher options (tuning / testing switches; no reference counterpart — the reference fixes
  * launch geometry in its bench drivers, bench.cu:375-636).  Names: "force_bn" (pin the tile width;
- * 0 = choose), "dense_pair", "sparse_pair" (0 = single-CTA kernels only), "row_balanced"
+ * 0 = choose; 240 and 224 select the CTA-pair kernels of sparse weights, tiles of 240 tokens, and of a sparse operand on
+ * the left, tiles of 256 columns), "dense_pair", "sparse_pair" (0 = single-CTA kernels only), "row_balanced"
  * (0 = whole 128-row tiles on the decode shapes), "tma_store" (0 = direct-store epilogue),
  * "dense_group_m", "sparse_col_first" (-1 automatic), "tail_narrow", "pdl", "gather_gbs",
  * "dense_decode" (dense weights [N x K], at most 256 tokens: -1 choose, 0 never / 1 always the kernel with

@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 # one-warp groups (several rows a CTA), groups of 1, 2 and 4 pieces a thread, rows longer than a group holds
 @pytest.mark.parametrize("M,K", [(1, 16), (3, 256), (149, 272), (150, 1024), (151, 1040), (148, 8192), (149, 8208), (200, 16384),
-                                 (150, 16400), (2, 32768), (3, 33040)])
+                                 (150, 16400), (2, 32768), (3, 33040), (149, 24592)])
 def test_all_group_sizes_match_the_reference_quantiser(M, K):
     rng = np.random.default_rng(M + 7 * K)
     x = (rng.standard_normal((M, K)) * np.exp2(rng.uniform(-14, 6, (M, 1)))).astype(np.float16)

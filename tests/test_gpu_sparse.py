@@ -240,8 +240,8 @@ def test_prune_to_2_4_matches_the_oracle_and_feeds_the_sparse_gemm(R, K):
 
 @pytest.mark.parametrize("M,N,K", [(256, 224, 256), (512, 448, 512), (144, 272, 1056), (400, 1008, 96), (1024, 2240, 2048)])
 def test_reference_orientation_on_cta_pairs(M, N, K):
-    """Sparse operand on the left, B[K x N], on CTA pairs (256 x 224 tiles; forced here, chosen by itself
-    for large shapes): exact int32 against the CPU GEMM of the decompressed matrix, ragged edges included,
+    """Sparse operand on the left, B[K x N], on CTA pairs (256 x 256 tiles; forced here, chosen by itself
+    where pairs need fewer waves): exact int32 against the CPU GEMM of the decompressed matrix, ragged edges included,
     and the fp32 reference ABI on top of the same integers."""
     dense, comp, meta, B = bench_sparse_inputs(M, N, K)
     want = oracle.igemm(dense, B, threads=0)
